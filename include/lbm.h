@@ -224,8 +224,10 @@ int   lbm_get_block(const lbm_ctx* c);
  * shared memory of one thread-block cluster: 128^2 FP32, 256^2 FP16S): the lattice stays resident in
  * the cluster's shared memory for up to 4096 steps of one launch, one cluster barrier per step, for
  * lattices too small to fill the GPU (a step is then launch-bound); lbm_step_planes and lone steps
- * inside CUDA graphs take PLAIN.  AUTO (default): the autotuner times the eligible ones.  All give
- * bit-identical results.                                                                            */
+ * inside CUDA graphs take PLAIN.  AUTO (default): the autotuner times the eligible ones; besides, runs of
+ * three and more steps of a D2Q9 BGK lattice advance several steps per launch, on overlapped tiles in
+ * shared memory, where that is faster (lattices that one wave of CTAs covers, and FP32 ones beyond L2).
+ * All give bit-identical results.                                                                   */
 enum lbm_kernel { LBM_KERNEL_AUTO = 0, LBM_KERNEL_PLAIN = 1, LBM_KERNEL_ROWS = 2, LBM_KERNEL_CLUSTER = 3 };
 int   lbm_set_kernel(lbm_ctx* c, int kind);
 int   lbm_get_kernel(const lbm_ctx* c);              /* the family in use (PLAIN, ROWS or CLUSTER), or AUTO before the first step */

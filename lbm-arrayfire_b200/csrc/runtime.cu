@@ -15,6 +15,7 @@
 #include "cluster.cuh"
 #include "kernels.cuh"
 #include "rowpipe.cuh"
+#include "tiles.cuh"
 
 namespace lbm {
 
@@ -129,6 +130,8 @@ struct lbm_ctx {
     int rows_grid = 0;             // persistent grid of the row pipeline (a whole step)
     int rows_per_sm = 0, sms = 0;  // its CTAs per SM and the device's SMs
     int reserved_sms = 0;          // lbm_set_reserved_sms: SMs the persistent grids leave free
+    TilePlan tiles;                // several steps per launch (tiles.cuh)
+    bool tune_block = true;        // the block width is left to the autotuner
     int cl_ctas = 0, cl_rows = 0;  // cluster-resident kernel: CTAs of the cluster, rows per CTA
     int rows_rpg = 1;              // its rows per group (segmented rows: the segment width)
     long long scw_target = 0;      // Shan-Chen window kernel: resident CTAs of the device (0: not queried)
@@ -632,6 +635,28 @@ static void launch_cluster(lbm_ctx* c, int from, cudaStream_t s, int k, bool wri
     });
 }
 
+// ---- several steps per launch on tiles (tiles.cu) ---------------------------------------------
+// D2Q9 BGK lattices whose kernel family is left to the engine, where the plan finds multi-step launches
+// faster; they own every SM, so not where some are reserved for other streams.
+static bool tiles_apply(const lbm_ctx* c) {
+    const lbm_desc& d = c->d;
+    return c->kernel == LBM_KERNEL_AUTO && c->tune_block && !c->reserved_sms && d.lattice == LBM_D2Q9 && d.collision == LBM_BGK &&
+           9ULL * (unsigned long long)c->N <= (1ULL << 32);
+}
+
+// One launch of T steps from buffer `from` into the other one.
+static cudaError_t launch_tiles(lbm_ctx* c, int from, cudaStream_t s, int T) {
+    TileLaunch l{};
+    l.pf = c->pf;
+    l.pd = c->pd;
+    l.err = c->err;
+    l.sms = c->sms;
+    l.pf.fin = l.pd.fin = c->f[from];
+    l.pf.fout = l.pd.fout = c->f[from ^ 1];
+    l.pf.parity = l.pd.parity = from;
+    return launch_tiles(c->d, l, c->tiles, T, s);
+}
+
 static std::mutex g_tune_mu;
 static std::map<std::string, int> g_tune_cache;
 
@@ -1020,7 +1045,18 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
     }
     LBM_CK(cudaEventRecord(c->e0, c->stream));
     long long n = nsteps;
-    if (c->kernel_used == LBM_KERNEL_CLUSTER) {
+    if (tiles_apply(c)) {
+        if (!c->sms) LBM_CK(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->d.device));
+        c->tiles = plan_tiles(c->d, c->sms);
+        // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
+        while (c->tiles.kind != kTilesNone && n > 2) {
+            const int k = (int)std::min<long long>((n - 1) / 2 * 2, c->tiles.steps);
+            LBM_CK(launch_tiles(c, c->cur, c->stream, k));
+            c->cur ^= 1;
+            n -= k;
+        }
+    }
+    if (c->kernel_used == LBM_KERNEL_CLUSTER && c->tiles.kind == kTilesNone) {
         while (n > 0) {
             const int k = (int)std::min<long long>(n, kClusterMaxSteps);
             launch_cluster(c, c->cur, c->stream, k);
@@ -1038,7 +1074,7 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
         c->cur ^= 1;
         --n;
     }
-    if (n >= 2) {
+    if (n > 2) {
         if (!c->gsteps) {
             int rc = build_graphs(c);
             if (rc) return rc;
@@ -1242,6 +1278,7 @@ int lbm_set_block(lbm_ctx* c, int threads_x) {
     LBM_CK(cudaStreamSynchronize(c->stream));
     drop_graphs(c);
     c->block = threads_x;
+    c->tune_block = threads_x == 0;
     c->kernel_used = 0;
     return LBM_OK;
 }
@@ -1268,7 +1305,10 @@ int lbm_set_kernel(lbm_ctx* c, int kind) {
     drop_graphs(c);
     c->kernel = kind;
     c->kernel_used = 0;
-    if (kind == LBM_KERNEL_ROWS || kind == LBM_KERNEL_CLUSTER) c->block = 0;
+    if (kind == LBM_KERNEL_ROWS || kind == LBM_KERNEL_CLUSTER) {
+        c->block = 0;
+        c->tune_block = true;
+    }
     return LBM_OK;
 }
 

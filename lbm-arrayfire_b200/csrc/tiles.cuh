@@ -1,0 +1,659 @@
+// tiles.cuh — several time steps of a D2Q9 BGK lattice per launch, on overlapped tiles in shared memory.
+//
+// A step of the one-step kernels reads and writes every population in HBM (or L2) and ends in a launch
+// boundary: large FP32 lattices are bound by HBM, small ones by the launch and its drain.  Here a CTA
+// advances a tile of W x h cells by T steps: it brings the tile and a halo of T cells into shared memory
+// once, collides T times on a region that shrinks by one cell per side and step, and stores the tile.
+// Populations cross HBM once per T steps instead of T times, for the redundant collisions in the halo
+// (1.2 per cell with 64 x 34 tiles and 4 steps).
+//
+// One copy of the populations is enough (the A-A pattern, Bailey et al. 2009).  A cell's populations lie at
+// its own index or, after every other step, at its neighbours': a step reads and writes the same nine words,
+// which no other cell touches in that step, so it needs no second buffer and one barrier.
+//   odd steps   read (x - c_i, i) = f_i's source,              write (x + c_i, opp(i)) <- f_i
+//   even steps  read (x, opp(i)) = what an odd step left,      write (x, i)            <- f_i
+//
+// Cells of the region are indexed flat, k = ly PX + lx, and a step walks whole rows: the outermost valid
+// cells give way to invalid ones by one cell per side and step, whatever those hold, so no column bounds are
+// tested in the loop.  A direction's words are contiguous and its place is a compile-time constant, so every
+// access is one register plus an immediate.
+//
+// The collision of two cells at a time in packed FP32 (add/mul/fma.f32x2) is what bounds the kernel: a packed
+// instruction does two cells' work in one issue slot and two cycles of the FP32 pipe.  A pair takes 109
+// packed instructions, 24-36 shared-memory accesses and some 20 others; a step of a 64 x 34 tile takes 3000 to
+// 3700 cycles where the FP32 pipe alone needs 2350 (scalar arithmetic: 209 instructions per cell, 110 GLUPS at
+// 4096^2 against 142).  The moves: 16-byte cp.async (.cg: past the small L1 that 227 KB of shared memory leave;
+// .ca took 710 us per 4 steps at 4096^2 against 540) while the lattice has one tile per SM; where SMs take
+// many tiles, four warps of their own move whole rows by bulk copies beside the computing ones (one warp
+// issues a bulk copy every 58 cycles, four keep up).
+//
+// Measured on B200 (us per step, one-step kernels -> tiles, lid cavities): 128^2 FP32 1.74 -> 0.85 and FP16S
+// 2.07 -> 1.06 (8 steps of 16 x 8 tiles); 1024 x 256 channel FP32 4.5 -> 3.5, FP16S 5.2 -> 4.2; 4096^2 FP32 188 ->
+// 118 (142 GLUPS; at one crossing per step HBM allows 91).
+//
+// The cell update is the other kernels' (bgk_collide, codecs and random words, with the step counter advanced
+// by T), so the results are bit-identical to single steps.  A launch leaves the state after T steps in
+// the other buffer and the state T steps earlier where it was, so the host ends every run with a single step
+// (lbm_get_macros and lbm_residual_fp64 read the state before the last one).
+#pragma once
+
+#include "internal.h"
+#include "rowpipe.cuh"
+
+namespace lbm {
+
+// ---- two cells at a time in packed FP32 arithmetic ------------------------------------------
+struct f32x2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 a, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ f32x2 both(float a) { return pack2(a, a); }
+__device__ __forceinline__ f32x2 operator+(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 operator-(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 operator*(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mad(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 neg(f32x2 a) { return f32x2{a.v ^ 0x8000000080000000ull}; }
+__device__ __forceinline__ float rcp_approx(float a) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+
+// 1 / a: the hardware's approximation and one Newton step in the form that rounds correctly (Markstein
+// 1990).  Equal to the division for every float with 2^-24 <= |a| < 2^126 (tested on all of them); NaN for
+// zero and infinite a, where a velocity j / rho is NaN either way.
+__device__ __forceinline__ f32x2 reciprocal(f32x2 a, f32x2 neg_a) {
+    float lo, hi;
+    unpack2(a, lo, hi);
+    const f32x2 r = pack2(rcp_approx(lo), rcp_approx(hi));
+    return mad(mad(neg_a, r, both(1.0f)), r, r);
+}
+
+// What a class overwrites, as the packed collision takes it (a table in shared memory).
+struct __align__(16) PairClass {
+    uint32_t fl;
+    float rho, ux, uy;
+};
+
+// bgk_collide of two D2Q9 cells at once (FP32 arithmetic on deviations v, in storage units): its operations
+// in its order, each on both lanes, so every lane's result is bgk_collide's.  A, B: the cells' classes
+// (SPECIAL; without it both are plain fluid).  No Zou-He cells.
+// minus_zero: a packed -0 the compiler cannot see through; with it a product that feeds an addition is a
+// multiply-add of the same value, which cannot be contracted into the addition.
+template <bool EXACTW, bool SPECIAL>
+__device__ __forceinline__ void bgk_pair(const StepParams<float>& p, const PairClass& A, const PairClass& B, f32x2 (&v)[9],
+                                         float sc, float isc, f32x2 minus_zero, f32x2 (&out)[9]) {
+    using L = D2Q9;
+    const f32x2 one = both(1.0f), isc2 = both(isc);
+    f32x2 r = v[0];
+    static_for<8>([&](auto I) { r = r + v[I + 1]; });
+    const f32x2 jx = ((((v[1] - v[3]) + v[5]) - v[6]) - v[7]) + v[8];
+    const f32x2 jy = ((((v[2] - v[4]) + v[5]) + v[6]) - v[7]) - v[8];
+    f32x2 drho = EXACTW ? r : r * isc2;
+    f32x2 rho = one + drho;
+    const f32x2 nrho = neg(rho);
+    const f32x2 rinv = reciprocal(rho, nrho);
+    const f32x2 inv = EXACTW ? rinv : rinv * isc2;  // a power of two: exact
+    auto quot = [&](f32x2 j) {
+        const f32x2 q = j * inv;
+        return mad(mad(q, nrho, EXACTW ? j : j * isc2), rinv, q);
+    };
+    f32x2 ux = quot(jx), uy = quot(jy);
+    if constexpr (SPECIAL) {
+        float a, b, c, d;
+        unpack2(rho, a, b);
+        unpack2(drho, c, d);
+        if (A.fl & kSetRho) a = A.rho, c = A.rho - 1.0f;
+        if (B.fl & kSetRho) b = B.rho, d = B.rho - 1.0f;
+        rho = pack2(a, b);
+        drho = pack2(c, d);
+        unpack2(ux, a, b);
+        if (A.fl & kSetUx) a = A.ux;
+        if (B.fl & kSetUx) b = B.ux;
+        ux = pack2(a, b);
+        unpack2(uy, a, b);
+        if (A.fl & kSetUy) a = A.uy;
+        if (B.fl & kSetUy) b = B.uy;
+        uy = pack2(a, b);
+    }
+    const f32x2 nusq15 = both(-1.5f) * mad(uy, uy, ux * ux);
+    const f32x2 rho3 = both(3.0f) * rho, rho45 = both(4.5f) * rho;
+    const f32x2 base = mad(rho, nusq15, drho);
+    const f32x2 om = both(p.omega), om1 = both(p.one_m_omega);
+    auto wmul = [&](auto I, f32x2 x) {
+        constexpr int i = decltype(I)::value;
+        if constexpr (EXACTW) {
+            constexpr float hi = float(L::w(i)), lo = float(L::w(i) - double(hi));
+            return mad(both(hi), x, both(lo) * x);
+        } else {
+            return mad(both(float(L::w(i)) * sc), x, minus_zero);
+        }
+    };
+    auto relax = [&](auto I, f32x2 fe) {
+        constexpr int i = decltype(I)::value;
+        f32x2 o = mad(om, fe, om1 * v[i]);
+        if constexpr (SPECIAL) {
+            float a, b, c, d;
+            unpack2(o, a, b);
+            unpack2(fe, c, d);
+            if (A.fl & kEquilibrium) a = c;
+            if (B.fl & kEquilibrium) b = d;
+            if constexpr (i > 0) {
+                unpack2(v[L::opp(i)], c, d);
+                if (A.fl & kBounce) a = c;
+                if (B.fl & kBounce) b = d;
+            }
+            o = pack2(a, b);
+        }
+        out[i] = o;
+    };
+    auto dirs = [&](auto I, f32x2 eu) {
+        constexpr int o = L::opp(decltype(I)::value);
+        const f32x2 sym = wmul(I, mad(rho45, eu * eu, base));
+        const f32x2 anti = wmul(I, rho3 * eu);
+        relax(I, sym + anti);
+        relax(std::integral_constant<int, o>{}, sym - anti);
+    };
+    relax(std::integral_constant<int, 0>{}, wmul(std::integral_constant<int, 0>{}, base));
+    dirs(std::integral_constant<int, 1>{}, ux);
+    dirs(std::integral_constant<int, 2>{}, uy);
+    dirs(std::integral_constant<int, 5>{}, ux + uy);
+    dirs(std::integral_constant<int, 6>{}, uy - ux);
+}
+
+// Shape of the tile kernel: source regions of up to MAXR rows of PX cells in shared memory, direction by
+// direction, HALO columns on either side of the tile's W.  MOVERS: warps that do nothing but bring the
+// next tile's region in and store the last one's tile (bulk copies; two buffers), 0: the computing warps do.
+// The steps compute the PW middle columns: T <= (PW - W) / 2.
+template <class S, int PX_, int PW_, int MAXR_, int HALO_, int WARPS_, int MOVERS_>
+struct TileShape {
+    using Word = S;
+    static constexpr int PX = PX_, PW = PW_, MAXR = MAXR_, HALO = HALO_, WARPS = WARPS_, MOVERS = MOVERS_;
+    static constexpr int kMaxSteps = (PW - (PX - 2 * HALO)) / 2;
+    static constexpr int NBUF = MOVERS > 0 ? 2 : 1;
+    static constexpr int W = PX - 2 * HALO, THREADS = 32 * WARPS, BLOCK = THREADS + 32 * MOVERS;
+    static constexpr int GUARD = 16 / (int)sizeof(S);  // words before and after a direction's region
+    static constexpr int PLANE = MAXR * PX + 2 * GUARD;
+    static constexpr int BUF = 9 * PLANE;
+    static_assert((PX * sizeof(S)) % 16 == 0 && (HALO * sizeof(S)) % 16 == 0, "rows of whole 16-byte words");
+    static constexpr size_t kPop = 64 + sizeof(PairClass) * kMaxClasses;
+    static constexpr size_t kCls = kPop + (size_t)NBUF * BUF * sizeof(S);
+    static constexpr size_t kClsBytes = (size_t)(MAXR * PX + 15) / 16 * 16;
+    static constexpr size_t smem_bytes() { return kCls + NBUF * kClsBytes; }
+};
+
+// How a lattice's multi-step launches are cut.
+enum TileKind { kTilesNone = 0, kTilesSmall, kTilesMid, kTilesStream };
+struct TilePlan {
+    int kind = kTilesNone;
+    int h = 0;      // rows of a tile (even)
+    int steps = 0;  // steps per launch (even)
+};
+struct TileLaunch {
+    StepParams<float> pf;
+    StepParams<double> pd;
+    int* err;
+    int sms;
+};
+// The plan of a D2Q9 BGK lattice on a device of `sms` SMs (kTilesNone: single steps are faster).
+TilePlan plan_tiles(const lbm_desc& d, int sms);
+cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int T, cudaStream_t s);
+
+// Two adjacent words.
+template <class S>
+struct __align__(2 * sizeof(S)) Two {
+    S a, b;
+};
+
+// A cell's byte in shared memory: class, and marks for a class with flags, a zero-gradient one, a Zou-He one.
+constexpr uint32_t kMarkFlags = 0x80u, kMarkOutlet = 0x40u, kMarkZouHe = 0x20u, kMarkClass = 0x0fu;
+// The same marks by class, one bit a class.
+struct ClassMarks {
+    uint32_t flags, outlet, zouhe;
+};
+
+__device__ __forceinline__ void bulk_store(void* dst_gmem, const void* src_smem, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst_gmem), "r"(smem_addr(src_smem)),
+                 "r"(bytes)
+                 : "memory");
+}
+
+// One tile launch: tiles of W x h cells, T (even, <= HALO) steps.  nx >= PX and ny >= h + 2 T
+// (host-checked): every region cell wraps at most once.  CTAs walk the tiles with a stride.  A thread takes
+// two cells at a time (PX and h are even).
+// G: bytes of the pieces that regions and tiles move in, 16, 8, 4 or (16-bit words) 2: every row of the
+// lattice starts on a multiple of it (16 with movers).
+template <class S, bool ABS, class Sh, int G>
+__global__ void __launch_bounds__(Sh::BLOCK, 1)
+    k_step_tiles(const __grid_constant__ StepParams<typename Codec<S>::Real> p, int h, int T, int tiles_x, int tiles,
+                 const ClassMarks marks, float minus_zero, int* __restrict__ err) {
+    using L = D2Q9;
+    using R = typename Codec<S>::Real;
+    constexpr int Q = 9, PX = Sh::PX, PLANE = Sh::PLANE, THREADS = Sh::THREADS, HALO = Sh::HALO, W = Sh::W, NBUF = Sh::NBUF;
+    constexpr bool k16 = Codec<S>::kScaled, kMove = Sh::MOVERS > 0;
+    constexpr bool kPacked = std::is_same_v<R, float> && !ABS;
+    extern __shared__ __align__(128) unsigned char smem[];
+    uint64_t* const full = reinterpret_cast<uint64_t*>(smem);  // movers: [NBUF] the region is there
+    uint64_t* const done = full + 2;                           // movers: [NBUF] the tile is computed
+    PairClass* const table = reinterpret_cast<PairClass*>(smem + 64);
+    S* const pops = reinterpret_cast<S*>(smem + Sh::kPop) + Sh::GUARD;
+    const int tid = (int)threadIdx.x;
+    const int nx = p.nx, ny = p.ny;
+    const int rows = h + 2 * T;  // of the source region
+    const uint32_t N = (uint32_t)p.N;  // 9 N <= 2^32 (host-checked)
+    const int stride = (int)gridDim.x;
+    constexpr int GW = G / (int)sizeof(S);  // cells of a piece
+    static_assert(GW >= 1 && GW * (int)sizeof(S) == G && (!kMove || G == 16), "pieces of whole words");
+    using Piece = std::conditional_t<G == 16, uint4, std::conditional_t<G == 8, uint2, std::conditional_t<G == 4, uint32_t, uint16_t>>>;
+
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid < kMaxClasses) table[tid] = PairClass{p.cls.flags[tid], (float)p.cls.rho[tid], (float)p.cls.ux[tid], (float)p.cls.uy[tid]};
+    if constexpr (kMove) {
+        if (tid == 0) {
+            for (int b = 0; b < NBUF; ++b) {
+                mbar_init(&full[b], 1);
+                mbar_init(&done[b], 1);
+            }
+            mbar_init_fence();
+        }
+        __syncthreads();
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the launch before this one is complete
+
+    const bool has_mask = p.mask != nullptr, words = has_mask && nx % 4 == 0;
+    auto mark = [&](uint32_t c) {
+        return c | ((marks.flags >> c) & 1u) << 7 | ((marks.outlet >> c) & 1u) << 6 | ((marks.zouhe >> c) & 1u) << 5;
+    };
+    auto cell_of = [&](int x0, int y0, int k) {  // lattice index of cell k of the region at (x0, y0)
+        const int ly = k / PX;
+        int x = x0 + (k - ly * PX), y = y0 + ly;
+        x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
+        y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+        return (uint32_t)y * (uint32_t)nx + (uint32_t)x;
+    };
+    // The region's class bytes, in words of four cells (x0 and PX are multiples of 4): a thread's words
+    // from global memory, and with their marks to shared memory (returns the marks among them).
+    constexpr int kClsWords = (Sh::MAXR * (PX / 4) + THREADS - 1) / THREADS;
+    auto get_classes = [&](int n, uint32_t (&c)[kClsWords]) {
+        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - T;
+        static_for<kClsWords>([&](auto J) {
+            const int j = tid + decltype(J)::value * THREADS;
+            c[J] = 0;
+            if (!has_mask || j >= rows * (PX / 4)) return;
+            if (words)
+                c[J] = __ldg(reinterpret_cast<const uint32_t*>(p.mask + cell_of(x0, y0, 4 * j)));
+            else
+                for (int u = 0; u < 4; ++u) c[J] |= (uint32_t)__ldg(p.mask + cell_of(x0, y0, 4 * j + u)) << (8 * u);
+        });
+    };
+    auto put_classes = [&](const uint32_t (&c)[kClsWords], int b) {
+        uint32_t* const dst = reinterpret_cast<uint32_t*>(smem + Sh::kCls + b * Sh::kClsBytes);
+        uint32_t seen = 0;
+        static_for<kClsWords>([&](auto J) {
+            const int j = tid + decltype(J)::value * THREADS;
+            if (j >= rows * (PX / 4)) return;
+            uint32_t w = 0;
+            for (int u = 0; u < 4; ++u) w |= mark((c[J] >> (8 * u)) & 0xffu) << (8 * u);
+            dst[j] = w;
+            seen |= w;
+        });
+        seen |= seen >> 16;
+        return (seen | seen >> 8) & (kMarkFlags | kMarkOutlet | kMarkZouHe);
+    };
+    const bool classes = has_mask || mark(0u) != 0;  // some cell of the lattice may not be plain fluid
+
+    if constexpr (kMove) {
+        if (tid >= THREADS) {
+            constexpr int MT = 32 * Sh::MOVERS;
+            const int m = tid - THREADS;
+            auto move_in = [&](int n, int b) {
+                const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - T;
+                const S* __restrict__ const fin = static_cast<const S*>(p.fin);
+                const int a = x0 < 0 ? x0 + nx : x0, len = nx - a < PX ? nx - a : PX;  // before the wrap in x
+                if (m == 0) mbar_arrive_expect_tx(&full[b], (uint32_t)(Q * rows * PX * (int)sizeof(S)));
+                for (int j = m; j < Q * rows; j += MT) {
+                    const int ly = j / Q, i = j - ly * Q;
+                    int y = y0 + ly;
+                    y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+                    const S* const row = fin + ((size_t)i * N + (size_t)((uint32_t)y * (uint32_t)nx));
+                    S* const dst = pops + b * Sh::BUF + i * PLANE + ly * PX;
+                    bulk_load(dst, row + a, (uint32_t)(len * (int)sizeof(S)), &full[b]);
+                    if (len < PX) bulk_load(dst + len, row, (uint32_t)((PX - len) * (int)sizeof(S)), &full[b]);
+                }
+            };
+            int n = (int)blockIdx.x;
+            for (int b = 0; b < NBUF; ++b)
+                if (n + b * stride < tiles) move_in(n + b * stride, b);
+            for (int turn = 0; n < tiles; ++turn, n += stride) {
+                const int b = turn & 1;
+                const bool ok = mbar_wait_bounded(&done[b], (uint32_t)((turn >> 1) & 1));
+                if (!ok) {
+                    atomicExch(err, kRowPipeTimeout);
+                    break;
+                }
+                const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W, y0 = ty * h;
+                const int w = nx - x0 < W ? nx - x0 : W, hh = ny - y0 < h ? ny - y0 : h;
+                S* const fout = static_cast<S*>(p.fout);
+                for (int j = m; j < Q * hh; j += MT) {
+                    const int r = j / Q, i = j - r * Q;
+                    bulk_store(fout + ((size_t)i * N + (size_t)((uint32_t)(y0 + r) * (uint32_t)nx + (uint32_t)x0)),
+                               pops + b * Sh::BUF + i * PLANE + (r + T) * PX + HALO, (uint32_t)(w * (int)sizeof(S)));
+                }
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                if (n + NBUF * stride < tiles) {
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    asm volatile("bar.sync 2, %0;" ::"n"(MT) : "memory");  // every mover's stores have read the buffer
+                    move_in(n + NBUF * stride, b);
+                }
+            }
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+            return;
+        }
+    }
+    auto barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); };
+    auto any = [](bool v) {
+        int r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(r)
+            : "r"((unsigned)v), "n"(THREADS)
+            : "memory");
+        return r != 0;
+    };
+
+    // The source region of tile n: f_i of cell (x0 + lx, y0 + ly) to [i][ly PX + lx].
+    auto move_in = [&](int n) {
+        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - T;
+        const char* const fin = static_cast<const char*>(p.fin);
+        for (int j = tid; j < rows * (PX / GW); j += THREADS) {
+            const int ly = j / (PX / GW), lx = (j - ly * (PX / GW)) * GW;
+            int x = x0 + lx, y = y0 + ly;
+            x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
+            y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+            const uint32_t off = ((uint32_t)y * (uint32_t)nx + (uint32_t)x) * (uint32_t)sizeof(S);
+            S* const dst = pops + ly * PX + lx;
+            static_for<Q>([&](auto I) {
+                constexpr int i = I;
+                const char* const base = fin + (size_t)i * N * sizeof(S);
+                if constexpr (G == 16)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst + i * PLANE)), "l"(base + off)
+                                 : "memory");
+                else if constexpr (G >= 4)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst + i * PLANE)), "l"(base + off),
+                                 "n"(G)
+                                 : "memory");
+                else
+                    dst[i * PLANE] = __ldcg(reinterpret_cast<const S*>(base + off));
+            });
+        }
+    };
+    // Tile n out.
+    auto move_out = [&](int n) {
+        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W, y0 = ty * h;
+        char* const fout = static_cast<char*>(p.fout);
+        const S* const buf = pops + T * PX + HALO;
+        for (int j = tid; j < h * (W / GW); j += THREADS) {
+            const int ly = j / (W / GW), lx = (j - ly * (W / GW)) * GW;
+            const int x = x0 + lx, y = y0 + ly;
+            if (x >= nx || y >= ny) continue;
+            const uint32_t off = ((uint32_t)y * (uint32_t)nx + (uint32_t)x) * (uint32_t)sizeof(S);
+            const S* const src = buf + ly * PX + lx;
+            static_for<Q>([&](auto I) {
+                constexpr int i = I;
+                char* const base = fout + (size_t)i * N * sizeof(S);
+                *reinterpret_cast<Piece*>(base + off) = *reinterpret_cast<const Piece*>(src + i * PLANE);
+            });
+        }
+    };
+
+    R sc, isc;
+    storage_scale<S>(p, sc, isc);
+    unsigned t0 = 0;
+    if constexpr (k16) {
+        if (p.sr) {
+            t0 = p.tick[p.parity];
+            if ((blockIdx.x | (unsigned)tid) == 0) p.tick[p.parity ^ 1] = t0 + (unsigned)T;
+        }
+    }
+    uint32_t next_cls[kClsWords], seen = 0;
+    if (kMove && classes && (int)blockIdx.x < tiles) {
+        get_classes((int)blockIdx.x, next_cls);
+        seen = put_classes(next_cls, 0);
+    }
+#pragma unroll 1
+    for (int turn = 0, n = (int)blockIdx.x; n < tiles; ++turn, n += stride) {
+        const int b = NBUF == 2 ? turn & 1 : 0;
+        const int ty = n / tiles_x, tx = n - ty * tiles_x;
+        const int x0 = tx * W - HALO, y0 = ty * h - T;
+        S* const pop = pops + b * Sh::BUF;
+        if constexpr (!kMove) move_in(n);
+        const uint8_t* const cls_s = smem + Sh::kCls + b * Sh::kClsBytes;
+        uint32_t kind = 0;  // marks among the region's cells
+        if constexpr (kMove) {
+            if (!mbar_wait_bounded(&full[b], (uint32_t)((turn >> 1) & 1))) {
+                atomicExch(err, kRowPipeTimeout);
+                return;
+            }
+        } else {
+            if (classes) {
+                get_classes(n, next_cls);
+                seen = put_classes(next_cls, 0);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+        }
+        if (classes) {
+            kind = any(seen != 0) ? kMarkFlags : 0u;
+            if (kind) kind |= (any((seen & kMarkOutlet) != 0) ? kMarkOutlet : 0u) | (any((seen & kMarkZouHe) != 0) ? kMarkZouHe : 0u);
+        } else if (!kMove) {
+            barrier();
+        }
+        // the next tile's classes travel while this one is computed
+        if (kMove && classes && n + stride < tiles) get_classes(n + stride, next_cls);
+
+        // One step.  AROUND (odd t): reads and writes the neighbours' words; else the cell's own.
+        auto step = [&](auto Around, auto Special, int t) {
+            constexpr bool around = decltype(Around)::value, SPECIAL = decltype(Special)::value;
+            Rounding rnd{0u, false};
+            if constexpr (k16) {
+                if (p.sr) rnd = Rounding{seed_of_step(t0 + (unsigned)(t - 1)), true};
+            }
+            // the two cells of a thread: adjacent, or (FP32 and FP64 words around, where adjacent cells would
+            // meet in a bank) half the rows apart
+            constexpr bool adj = !around || k16;
+            constexpr int PW = Sh::PW;
+            const int half = (rows / 2 - t) * PX;
+            const int count = (rows / 2 - t) * PW, second = adj ? 1 : half;  // pairs of cells
+            const int first = t * PX;
+            if constexpr (SPECIAL) {
+                // A zero-gradient cell's c_x = -1 populations are f_i(x, y - c_iy) of its own column, which
+                // the cell to its left reads and overwrites.  They are copied to where the cell itself
+                // reads, which no other cell touches in this step.
+                if (kind & kMarkOutlet) {
+                    const int w0 = first / 4, w1 = (rows * PX - first) / 4;
+                    for (int base = w0; base < w1; base += THREADS) {
+                        const int m = base + tid;
+                        const uint32_t word = m < w1 ? reinterpret_cast<const uint32_t*>(cls_s)[m] : 0u;
+                        const bool mine = (word & (kMarkOutlet * 0x01010101u)) != 0;
+                        S zg[4][3];
+                        if (mine) {
+                            static_for<4>([&](auto U) {
+                                static_for<3>([&](auto J) {
+                                    constexpr int u = U, i = J == 0 ? 3 : (J == 1 ? 6 : 7);
+                                    const int k = 4 * m + u;
+                                    zg[u][J] = around ? pop[i * PLANE + k - L::cy(i) * PX] : pop[L::opp(i) * PLANE + k - 1];
+                                });
+                            });
+                        }
+                        barrier();
+                        if (mine) {
+                            static_for<4>([&](auto U) {
+                                constexpr int u = U;
+                                if ((word >> (8 * u)) & kMarkOutlet)
+                                    static_for<3>([&](auto J) {
+                                        constexpr int i = J == 0 ? 3 : (J == 1 ? 6 : 7);
+                                        const int k = 4 * m + u;
+                                        (around ? pop[i * PLANE + k - L::cy(i) * PX + 1] : pop[L::opp(i) * PLANE + k]) = zg[u][J];
+                                    });
+                            });
+                        }
+                        barrier();
+                    }
+                }
+            }
+#pragma unroll 1
+            for (int j = tid; j < count; j += THREADS) {
+                int k = first + (adj ? 2 * j : j);
+                if constexpr (PW < PX) {
+                    constexpr int PR = adj ? PW / 2 : PW;  // pairs of a row
+                    k += (j / PR) * (PX - PW) + (PX - PW) / 2;
+                }
+                S* const c = pop + k;
+                S* const d = c + second;
+                S wA[Q], wB[Q];
+                static_for<Q>([&](auto I) {
+                    constexpr int i = I, o = around ? i * PLANE - (L::cy(i) * PX + L::cx(i)) : L::opp(i) * PLANE;
+                    if constexpr (adj && (!around || L::cx(i) == 0)) {
+                        const Two<S> w = *reinterpret_cast<const Two<S>*>(c + o);
+                        wA[i] = w.a;
+                        wB[i] = w.b;
+                    } else {
+                        wA[i] = c[o];
+                        wB[i] = d[o];
+                    }
+                });
+                uint32_t mA = 0, mB = 0;
+                if constexpr (SPECIAL) {
+                    mA = cls_s[k];
+                    mB = cls_s[k + second];
+                }
+                auto value = [&](S w, auto I) -> R {
+                    if constexpr (ABS)
+                        return R(w);
+                    else
+                        return Codec<S>::raw(w, R(L::w(decltype(I)::value)));
+                };
+                R oA[Q], oB[Q];  // stored values: collided deviations for the 16-bit codecs, populations else
+                auto scalar = [&](const S(&w)[Q], uint32_t m, R(&o)[Q]) {
+                    R v[Q], out[Q];
+                    const int cls = (int)(m & kMarkClass);
+                    static_for<Q>([&](auto I) { v[I] = value(w[I], I); });
+                    bgk_collide<L, ABS, kExactWeights<S>>(p, cls, SPECIAL ? p.cls.flags[cls] : 0u, v, sc, isc, out);
+                    static_for<Q>([&](auto I) {
+                        constexpr int i = I;
+                        if constexpr (k16 || ABS)
+                            o[i] = out[i];
+                        else
+                            o[i] = Codec<S>::enc(out[i], R(L::w(i)));
+                    });
+                };
+                if constexpr (kPacked) {
+                    auto packed = [&](auto Sp) {
+                        f32x2 v[Q], out[Q];
+                        static_for<Q>([&](auto I) {
+                            constexpr int i = I;
+                            if constexpr (k16)
+                                v[i] = pack2(value(wA[i], I), value(wB[i], I));
+                            else
+                                v[i] = pack2(wA[i], wB[i]) - both(float(L::w(i)));
+                        });
+                        PairClass A{}, B{};
+                        if constexpr (decltype(Sp)::value) {
+                            A = table[mA & kMarkClass];
+                            B = table[mB & kMarkClass];
+                        }
+                        bgk_pair<kExactWeights<S>, decltype(Sp)::value>(p, A, B, v, sc, isc, both(minus_zero), out);
+                        static_for<Q>([&](auto I) {
+                            constexpr int i = I;
+                            // F32: the stored word w + d
+                            unpack2(k16 ? out[i] : both(float(L::w(i))) + out[i], oA[i], oB[i]);
+                        });
+                    };
+                    if constexpr (!SPECIAL) {
+                        packed(std::false_type{});
+                    } else if (!__any_sync(__activemask(), ((mA | mB) & kMarkFlags) != 0u)) {
+                        packed(std::false_type{});
+                    } else if (kind & kMarkZouHe) {
+                        scalar(wA, mA, oA);
+                        scalar(wB, mB, oB);
+                    } else {
+                        packed(std::true_type{});
+                    }
+                } else {
+                    scalar(wA, mA, oA);
+                    scalar(wB, mB, oB);
+                }
+                // stored words
+                if constexpr (k16) {
+                    // the same random bits as encode16 gives each cell, both cells of a direction in one conversion
+                    const uint32_t cA = cell_of(x0, y0, k) + p.cell_base, cB = cell_of(x0, y0, k + 1) + p.cell_base;
+                    const PairBits pb{(cell_hash16(cB, rnd.seed) << 16) | cell_hash16(cA, rnd.seed)};
+                    static_for<Q>([&](auto I) {
+                        constexpr int i = I, o = around ? L::opp(i) * PLANE + (L::cy(i) * PX + L::cx(i)) : i * PLANE;
+                        const uint32_t w = rnd.sr ? Pair16<S>::rs(oB[i], oA[i], pb.template word<i, i>()) : Pair16<S>::rn(oB[i], oA[i]);
+                        if constexpr (!around || L::cx(i) == 0) {
+                            *reinterpret_cast<uint32_t*>(c + o) = w;
+                        } else {
+                            c[o] = Pair16<S>::lo(w);
+                            d[o] = Pair16<S>::hi(w);
+                        }
+                    });
+                } else {
+                    static_for<Q>([&](auto I) {
+                        constexpr int i = I, o = around ? L::opp(i) * PLANE + (L::cy(i) * PX + L::cx(i)) : i * PLANE;
+                        if constexpr (adj) {
+                            *reinterpret_cast<Two<S>*>(c + o) = Two<S>{S(oA[i]), S(oB[i])};
+                        } else {
+                            c[o] = S(oA[i]);
+                            d[o] = S(oB[i]);
+                        }
+                    });
+                }
+            }
+            if (kMove && !around && t == T) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            barrier();
+        };
+        auto steps = [&](auto Special) {
+#pragma unroll 1
+            for (int t = 1; t < T; t += 2) {
+                step(std::true_type{}, Special, t);
+                step(std::false_type{}, Special, t + 1);
+            }
+        };
+        if (kind)
+            steps(std::true_type{});
+        else
+            steps(std::false_type{});
+        if constexpr (kMove) {
+            if (tid == 0) mbar_arrive(&done[b]);
+            if (classes && n + stride < tiles) seen = put_classes(next_cls, b ^ 1);
+        } else {
+            move_out(n);
+            if (n + stride < tiles) barrier();
+        }
+    }
+}
+
+}  // namespace lbm
