@@ -1071,15 +1071,18 @@ __global__ void __launch_bounds__(kScwTX, sizeof(typename Codec<S>::Real) == 8 ?
 // ---- macroscopic fields ------------------------------------------------------------------
 // pulled = 1: the fields the last step's collision used (pull from the previous buffer, class
 // overwrites, Shan-Chen velocity u + F/(2 rho)).  pulled = 0: local moments of p.fin.
-template <class L, class S, class O>
-__global__ void k_macros(const __grid_constant__ StepParams<typename Codec<S>::Real> p, int pulled, int collision, O* rho_out,
-                         O* u_out) {
+// I32: 32-bit population indices (lattices with Q N <= 2^32), as in the step kernels (256^3 D3Q27 FP16S 383 ->
+// 254 us, (251, 83, 83) 53 -> 40).
+template <class L, class S, class O, bool I32>
+__global__ void __launch_bounds__(128) k_macros(const __grid_constant__ StepParams<typename Codec<S>::Real> p, int pulled,
+                                                int collision, O* rho_out, O* u_out) {
     using R = typename Codec<S>::Real;
+    using Ix = typename std::conditional<I32, uint32_t, long long>::type;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= p.nx) return;
     const int y = blockIdx.y, z = blockIdx.z;
-    const Rows<L> rows(y, z, p.nx, p.ny, p.nz);
-    const long long c = rows.base[1][1] + x;
+    const RowsT<L, Ix> rows(y, z, p.nx, p.ny, p.nz);
+    const Ix c = rows.base[1][1] + (Ix)x;
     const S* __restrict__ fin = static_cast<const S*>(p.fin);
     R d[L::Q];
     int cls;
@@ -1091,7 +1094,7 @@ __global__ void k_macros(const __grid_constant__ StepParams<typename Codec<S>::R
     } else {
         static_for<L::Q>([&](auto I) {
             constexpr int i = I;
-            d[i] = Codec<S>::raw(__ldg(fin + (long long)i * p.N + c), R(L::w(i)));
+            d[i] = Codec<S>::raw(__ldg(fin + ((Ix)i * (Ix)p.N + c)), R(L::w(i)));
         });
     }
     R sc, isc;
@@ -1181,12 +1184,16 @@ __global__ void __launch_bounds__(256) k_sums_partial(const S* __restrict__ f, l
     }
 }
 
-// Stage 2: one thread folds the partials in index order.
+// Stage 2: one block folds the partials (defined in runtime.cu).
+constexpr int kFoldThreads = 256;
 __global__ void k_sums_final(const Sums* __restrict__ partial, int n, Sums* __restrict__ out);
 
-// Residual partials: sum |u_a - u_b|^2 and |u_a|^2 over class-0 cells (local moments).
+// Residual partials: sum |u_a - u_b|^2 and |u_a|^2 over class-0 cells (local moments).  FP64 arithmetic
+// bounds it (two conversions and six adds a direction): the momenta take adds only, no products with the
+// velocity's -1, 0, 1, one reciprocal per state, and D3Q27 keeps four blocks an SM (it took 210 registers
+// unbounded).  lbm_residual_fp64, with the fold: 256^3 D3Q27 FP32 3.17 -> 1.06 ms, 4096^2 D2Q9 FP32 1.03 -> 0.32.
 template <class L, class S>
-__global__ void __launch_bounds__(256) k_residual_partial(const S* __restrict__ fa, const S* __restrict__ fb,
+__global__ void __launch_bounds__(256, L::DIM == 3 ? 4 : 2) k_residual_partial(const S* __restrict__ fa, const S* __restrict__ fb,
                                                            const uint8_t* __restrict__ mask, long long N,
                                                            float inv_scale, Sums* __restrict__ partial) {
     using R = typename Codec<S>::Real;
@@ -1197,20 +1204,23 @@ __global__ void __launch_bounds__(256) k_residual_partial(const S* __restrict__ 
         double ra = 0, xa = 0, ya = 0, za = 0, rb = 0, xb = 0, yb = 0, zb = 0;
         static_for<L::Q>([&](auto I) {
             constexpr int i = I;
+            constexpr int cx = L::cx(i), cy = L::cy(i), cz = L::cz(i);
             const double a = (double)Codec<S>::load(fa + (long long)i * N + c, R(L::w(i)), R(inv_scale));
             const double b = (double)Codec<S>::load(fb + (long long)i * N + c, R(L::w(i)), R(inv_scale));
             ra += a;
             rb += b;
-            xa += L::cx(i) * a;
-            xb += L::cx(i) * b;
-            ya += L::cy(i) * a;
-            yb += L::cy(i) * b;
-            za += L::cz(i) * a;
-            zb += L::cz(i) * b;
+            if constexpr (cx == 1) xa += a, xb += b;
+            if constexpr (cx == -1) xa -= a, xb -= b;
+            if constexpr (cy == 1) ya += a, yb += b;
+            if constexpr (cy == -1) ya -= a, yb -= b;
+            if constexpr (cz == 1) za += a, zb += b;
+            if constexpr (cz == -1) za -= a, zb -= b;
         });
-        const double dx = xa / ra - xb / rb, dy = ya / ra - yb / rb, dz = za / ra - zb / rb;
+        const double ia = 1.0 / ra, ib = 1.0 / rb;
+        const double ux = xa * ia, uy = ya * ia, uz = za * ia;
+        const double dx = ux - xb * ib, dy = uy - yb * ib, dz = uz - zb * ib;
         num += dx * dx + dy * dy + dz * dz;
-        den += (xa * xa + ya * ya + za * za) / (ra * ra);
+        den += ux * ux + uy * uy + uz * uz;
     }
     __shared__ double sh[2][8];
     num = warp_sum(num);

@@ -90,7 +90,7 @@ extern "C" int lbm_sums_fp64_noalloc(const void* populations, int lattice, int s
         k_sums_partial<L, S><<<blocks, kThreads, 0, s>>>(static_cast<const S*>(populations), N,
                                                          (float)(1.0 / scale), scratch);
     });
-    k_sums_final<<<1, 32, 0, s>>>(scratch, blocks, scratch + kMaxPartials);
+    k_sums_final<<<1, kFoldThreads, 0, s>>>(scratch, blocks, scratch + kMaxPartials);
     LBM_CK(cudaGetLastError());
     Sums r;
     LBM_CK(cudaMemcpyAsync(&r, scratch + kMaxPartials, sizeof(Sums), cudaMemcpyDeviceToHost, s));
