@@ -657,7 +657,7 @@ static void launch_cluster(lbm_ctx* c, int from, cudaStream_t s, int k, bool wri
 // faster; they own every SM, so not where some are reserved for other streams.
 static bool tiles_apply(const lbm_ctx* c) {
     const lbm_desc& d = c->d;
-    return c->kernel == LBM_KERNEL_AUTO && c->tune_block && !c->reserved_sms && d.lattice == LBM_D2Q9 && d.collision == LBM_BGK &&
+    return c->kernel == LBM_KERNEL_AUTO && c->tune_block && !c->reserved_sms && d.lattice == LBM_D2Q9 && d.collision != LBM_MRT &&
            9ULL * (unsigned long long)c->N <= (1ULL << 32);
 }
 

@@ -8,24 +8,30 @@
 namespace lbm {
 
 // The shapes.  Region rows start on 16-byte words, so the halo is 4 columns for FP32 and FP64 and 8 for
-// 16-bit words.  Small: tiles of 16 columns, up to 8 steps; mid: 64 columns, up to 4 steps, one region;
-// stream: mid with two regions and four moving warps.
+// 16-bit words.  Small: tiles of 16 columns, up to 8 steps; mid: 64 columns, up to 4 steps, one region; pieces,
+// stream: mid with two regions and four moving warps.  Bulk copies do not occupy the load/store units while HBM
+// answers, but take some 20 issue slots each: they win where the populations stream from HBM (4096^2 FP32 113 us a
+// step against 126 in pieces, 2048 x 1024 19.2 against 20.5), pieces where they stay in L2 (1024^2 10.6 against
+// 11.2) and for Shan-Chen's two steps a launch (1024^2 15.1 against 17.5).
 template <class S>
 constexpr int kMidHalo = sizeof(S) == 2 ? 8 : 4;
 template <class S>
-using SmallShape = TileShape<S, 32, 32, 24, 8, 12, 0>;
+using SmallShape = TileShape<S, false, 32, 32, 24, 8, 12, 0, false>;
 template <class S>
-using MidShape = TileShape<S, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 8 ? 40 : 44, kMidHalo<S>, sizeof(S) == 8 ? 16 : 24, 0>;
+using MidShape = TileShape<S, false, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 8 ? 40 : 44, kMidHalo<S>, sizeof(S) == 8 ? 16 : 24, 0, false>;
+template <class S, bool BULK>
+using StreamShape =
+    TileShape<S, false, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 8 ? 20 : 42, kMidHalo<S>, sizeof(S) == 8 ? 12 : 20, 4, BULK>;
 template <class S>
-using StreamShape = TileShape<S, 64 + 2 * kMidHalo<S>, 72, 42, kMidHalo<S>, 20, 4>;
+using ShanChenShape = TileShape<S, true, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 2 ? 44 : 40, kMidHalo<S>, 20, 4, false>;
 
 template <class S, bool ABS, class Sh, int G>
 static cudaError_t launch_one(const StepParams<typename Codec<S>::Real>& p, const TileLaunch& l, const TilePlan& plan, int T,
                               cudaStream_t s) {
     static_assert(Sh::smem_bytes() <= 227 * 1024, "a tile's regions must fit into shared memory");
     // what the kernel's indices rely on
-    const bool fits = T >= 2 && T % 2 == 0 && T <= Sh::kMaxSteps && T <= Sh::HALO && plan.h >= 2 && plan.h % 2 == 0 &&
-                      plan.h + 2 * T <= Sh::MAXR && p.nx >= Sh::PX && p.ny >= plan.h + 2 * T &&
+    const bool fits = T >= 2 && T % 2 == 0 && T <= Sh::kMaxSteps && plan.h >= 2 && plan.h % 2 == 0 &&
+                      plan.h + 2 * Sh::D * T <= Sh::MAXR && p.nx >= Sh::PX && p.ny >= plan.h + 2 * Sh::D * T &&
                       ((size_t)p.nx * sizeof(S)) % G == 0 && 9ULL * (unsigned long long)p.N <= (1ULL << 32);
     if (!fits) return cudaErrorInvalidValue;
     auto kern = k_step_tiles<S, ABS, Sh, G>;
@@ -39,6 +45,7 @@ static cudaError_t launch_one(const StepParams<typename Codec<S>::Real>& p, cons
         marks.outlet |= (fl & kZeroGradXp ? 1u : 0u) << k;
         marks.zouhe |= (fl & (kZouHeVelXm | kZouHeRhoXp) ? 1u : 0u) << k;
     }
+    if (Sh::SC && marks.outlet) return cudaErrorInvalidValue;  // no zero-gradient cells in Shan-Chen tiles
     // a launch may be scheduled while the one before it drains (the kernel waits for its end itself)
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -61,7 +68,7 @@ static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, con
     // the largest pieces that every row starts on
     auto by_piece = [&](auto sh) {
         using Sh = decltype(sh);
-        if constexpr (kWord == 2 || (kWord == 4 && !ABS)) {
+        if constexpr (kWord == 2 || !ABS) {
             if (row % 16 == 0) return launch_one<S, ABS, Sh, 16>(p, l, plan, T, s);
         }
         if constexpr (kWord == 2) {
@@ -69,11 +76,18 @@ static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, con
         }
         return launch_one<S, ABS, Sh, kWord>(p, l, plan, T, s);
     };
-    if (plan.kind == kTilesSmall) return by_piece(SmallShape<S>{});
-    if constexpr (kWord == 4 && !ABS) {
-        if (plan.kind == kTilesStream && row % 16 == 0) return launch_one<S, ABS, StreamShape<S>, 16>(p, l, plan, T, s);
+    if constexpr (kWord <= 4 && !ABS) {
+        if (plan.kind == kTilesShanChen) return by_piece(ShanChenShape<S>{});
     }
-    return by_piece(MidShape<S>{});
+    if constexpr (kWord >= 4 && !ABS) {
+        if (plan.kind == kTilesStream && row % 16 == 0) return launch_one<S, ABS, StreamShape<S, true>, 16>(p, l, plan, T, s);
+    }
+    if constexpr (kWord == 4 && !ABS) {
+        if (plan.kind == kTilesPieces) return by_piece(StreamShape<S, false>{});
+    }
+    if (plan.kind == kTilesSmall) return by_piece(SmallShape<S>{});
+    if (plan.kind == kTilesMid) return by_piece(MidShape<S>{});
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int T, cudaStream_t s) {
@@ -89,40 +103,64 @@ cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan&
 }
 
 // When tiles are faster than single steps (measured on B200, lid cavities, us per step, single -> tiles).
-// - Lattices that one wave of CTAs covers: a launch of T steps then costs about 2 us of launch and drain, 2 us of
+// - BGK lattices that one wave of CTAs covers: a launch of T steps then costs about 2 us of launch and drain, 2 us of
 //   moves and T short steps.  Small tiles first, for more CTAs: 96^2 FP32 1.4 -> 0.9, 128^2 1.8 -> 1.0, 192^2
 //   (16-row tiles, 4 steps) 3.5 -> 1.5; then 64-column tiles: 256^2 4.7 -> 1.8, 512^2 4.6 -> 3.5, 1000 x 300 5.0 ->
 //   3.7 (FP16S 512^2 6.2 -> 4.0, 1000 x 300 5.0 -> 4.3).  FP64 collisions take twice as long, so only up to
 //   14 rows: 256^2 4.1 -> 2.7, 384^2 (16 rows) 4.3 -> 4.2, 512^2 5.3 -> 6.3.
-// - Two or three waves: nothing to gain (1024 x 512 FP32 6.6 -> 6.4, FP16S 7.4 -> 7.2; 1024^2 11.2 -> 11.9).
-// - FP32 lattices whose two buffers leave L2: streamed tiles, from about 80 MB (75 MB 11.2 -> 11.9, 86 MB 13.6 ->
-//   11.8, 118 MB 18.8 -> 16.7, 302 MB 49 -> 35); rows that do not start on 16-byte words cannot be moved in bulk
-//   and take the mid shape, from 125 MB (118 MB 18.8 -> 19.6, 122 MB 22.7 -> 20.0, 3001 x 2003 75.6 -> 68.6).
-//   16-bit words cross HBM fast enough in single steps (2048^2 FP16S 39.6 -> 46.6), FP64 gains 4 % at most.
+// - FP32 BGK in L2, several waves: a wave of h-row tiles takes 2.3 (h + 6) / 36 us, a launch 1.4, a single step 1.5
+//   and its cells at 107 G/s, which decides (1024 x 512 6.6 -> 6.2, 1024^2 11.2 -> 10.6; 1500 x 451 8.0 -> 8.7 stays
+//   single).  16-bit words gain nothing there (1024 x 512 FP16S 7.4 -> 7.2, 1024^2 11.4 -> 13.3).
+// - BGK lattices whose two buffers leave L2: FP32 from about 80 MB (75 MB 11.2 -> 11.9, 86 MB 13.6 -> 11.8, 151 MB
+//   26.3 -> 19.2, 433 MB 70 -> 45; rows that start anywhere move in pieces, from 125 MB: 433 MB 76 -> 63), FP64 with
+//   rows of whole 16-byte words from 140 MB (151 MB 24.0 -> 22.4, 302 MB 47 -> 39, 865 MB 132 -> 104; in pieces 134 ->
+//   137).  16-bit words cross HBM fast enough in single steps (2048^2 FP16S 39.6 -> 46.6).
+// - Shan-Chen, FP32 of any width and 16-bit words in rows of whole 16-byte words (in 2-byte pieces 2049 x 1537
+//   60.8 -> 73): FP32 256^2 8.3 -> 3.9, 1024^2 21.4 -> 15.1, 2049 x 1537 64 -> 54, 4096^2 298 -> 211; BF16S 8.2 -> 4.0,
+//   22.4 -> 15.8, 4096^2 291 -> 230.  A wave takes about h + 4 rows' time, so the height is the one whose waves times
+//   that is least (1024^2: 28 rows, 4.0 waves, 15.1; 32 rows, 3.5 waves, 17.0).
 TilePlan plan_tiles(const lbm_desc& d, int sms) {
     const bool abs_arith = d.arithmetic == LBM_ARITH_ABSOLUTE;
     const int word = storage_bytes(d.storage);
+    const bool whole = d.nx * word % 16 == 0;  // rows of whole 16-byte words
+    const int mid_px = 64 + 2 * (word == 2 ? 8 : 4);
+    auto tiles = [&](int w, int h) { return ((d.nx + w - 1) / w) * ((d.ny + h - 1) / h); };
+    auto waves = [&](int h) { return (tiles(64, h) + sms - 1) / sms; };
     // the smallest even height (at most `most`) at which tiles of w columns are no more than the SMs, or 0
     auto one_wave = [&](int w, int most) {
-        const long long tx = (d.nx + w - 1) / w;
         for (int h = 2; h <= most; h += 2)
-            if (tx * ((d.ny + h - 1) / h) <= sms) return h;
+            if (tiles(w, h) <= sms) return h;
         return 0;
     };
-    auto plan = [&](TileKind k, int px, int h, int steps) {
-        TilePlan t{};
-        if (h > 0 && d.nx >= px && d.ny >= h + 2 * steps) t = TilePlan{k, h, steps};
-        return t;
+    // the height with the shortest waves in all, a wave taking as long as h + over rows
+    auto best_height = [&](int most, int over) {
+        int best = 2;
+        for (int h = 4; h <= most; h += 2)
+            if (waves(h) * (h + over) < waves(best) * (best + over)) best = h;
+        return best;
     };
-    const int mid_px = 64 + 2 * (word == 2 ? 8 : 4);
-    if (const int h = one_wave(16, 8)) return plan(kTilesSmall, 32, h, 8);
-    if (const int h = one_wave(16, 16)) return plan(kTilesSmall, 32, h, 4);
-    if (const int h = one_wave(64, word == 8 ? 14 : 36)) return plan(kTilesMid, mid_px, h, 4);
-    const long long bytes = 2LL * 9 * word * d.nx * d.ny;  // both buffers
-    if (word == 4 && !abs_arith) {
-        if (d.nx % 4 == 0 && bytes > 80000000LL) return plan(kTilesStream, mid_px, 34, 4);
-        if (bytes > 125000000LL) return plan(kTilesMid, mid_px, 34, 4);
+    auto plan = [&](TileKind k, int px, int h, int steps, int depth) {
+        return d.nx >= px && d.ny >= h + 2 * depth ? TilePlan{k, h, steps} : TilePlan{};
+    };
+    if (d.collision == LBM_SHANCHEN) {
+        bool outlet = false;
+        for (int k = 0; k < d.n_classes; ++k) outlet = outlet || (d.classes[k].flags & LBM_CELL_ZEROGRAD_XP);
+        if (abs_arith || word == 8 || outlet || (word == 2 && !whole)) return TilePlan{};
+        return plan(kTilesShanChen, mid_px, best_height(word == 2 ? 36 : 32, 4), 2, 4);
     }
+    if (const int h = one_wave(16, 8)) return plan(kTilesSmall, 32, h, 8, 8);
+    if (const int h = one_wave(16, 16)) return plan(kTilesSmall, 32, h, 4, 4);
+    if (const int h = one_wave(64, word == 8 ? 14 : 36)) return plan(kTilesMid, mid_px, h, 4, 4);
+    if (abs_arith) return TilePlan{};
+    const long long bytes = 2LL * 9 * word * d.nx * d.ny;  // both buffers
+    if (word == 4 && whole && bytes > 80000000LL) return plan(kTilesStream, mid_px, 34, 4, 4);
+    if (word == 4 && !whole && bytes > 125000000LL) return plan(kTilesPieces, mid_px, 34, 4, 4);
+    if (word == 4 && whole) {
+        const int h = best_height(34, 6);
+        const double tiled = 1.4 + 2.3 / 36 * (double)(waves(h) * (h + 6)), single = 1.5 + (double)(d.nx * d.ny) / 107e3;
+        if (tiled < 0.97 * single) return plan(kTilesPieces, mid_px, h, 4, 4);
+    }
+    if (word == 8 && whole && bytes > 140000000LL) return plan(kTilesStream, mid_px, 12, 4, 4);
     return TilePlan{};
 }
 

@@ -98,22 +98,17 @@ struct __align__(16) PairClass {
     float rho, ux, uy;
 };
 
-// bgk_collide of two D2Q9 cells at once (FP32 arithmetic on deviations v, in storage units): its operations
-// in its order, each on both lanes, so every lane's result is bgk_collide's.  A, B: the cells' classes
-// (SPECIAL; without it both are plain fluid).  No Zou-He cells.
-// minus_zero: a packed -0 the compiler cannot see through; with it a product that feeds an addition is a
-// multiply-add of the same value, which cannot be contracted into the addition.
+// moments() and apply_class() of two cells.
 template <bool EXACTW, bool SPECIAL>
-__device__ __forceinline__ void bgk_pair(const StepParams<float>& p, const PairClass& A, const PairClass& B, f32x2 (&v)[9],
-                                         float sc, float isc, f32x2 minus_zero, f32x2 (&out)[9]) {
-    using L = D2Q9;
-    const f32x2 one = both(1.0f), isc2 = both(isc);
+__device__ __forceinline__ void pair_moments(const PairClass& A, const PairClass& B, const f32x2 (&v)[9], float isc, f32x2& rho,
+                                             f32x2& drho, f32x2& ux, f32x2& uy) {
+    const f32x2 isc2 = both(isc);
     f32x2 r = v[0];
     static_for<8>([&](auto I) { r = r + v[I + 1]; });
     const f32x2 jx = ((((v[1] - v[3]) + v[5]) - v[6]) - v[7]) + v[8];
     const f32x2 jy = ((((v[2] - v[4]) + v[5]) + v[6]) - v[7]) - v[8];
-    f32x2 drho = EXACTW ? r : r * isc2;
-    f32x2 rho = one + drho;
+    drho = EXACTW ? r : r * isc2;
+    rho = both(1.0f) + drho;
     const f32x2 nrho = neg(rho);
     const f32x2 rinv = reciprocal(rho, nrho);
     const f32x2 inv = EXACTW ? rinv : rinv * isc2;  // a power of two: exact
@@ -121,7 +116,8 @@ __device__ __forceinline__ void bgk_pair(const StepParams<float>& p, const PairC
         const f32x2 q = j * inv;
         return mad(mad(q, nrho, EXACTW ? j : j * isc2), rinv, q);
     };
-    f32x2 ux = quot(jx), uy = quot(jy);
+    ux = quot(jx);
+    uy = quot(jy);
     if constexpr (SPECIAL) {
         float a, b, c, d;
         unpack2(rho, a, b);
@@ -139,10 +135,15 @@ __device__ __forceinline__ void bgk_pair(const StepParams<float>& p, const PairC
         if (B.fl & kSetUy) b = B.uy;
         uy = pack2(a, b);
     }
+}
+
+// equilibrium_dev() of two cells: put(i, fe_i).
+template <bool EXACTW, class Put>
+__device__ __forceinline__ void pair_equilibrium(f32x2 rho, f32x2 drho, f32x2 ux, f32x2 uy, float sc, f32x2 minus_zero, Put&& put) {
+    using L = D2Q9;
     const f32x2 nusq15 = both(-1.5f) * mad(uy, uy, ux * ux);
     const f32x2 rho3 = both(3.0f) * rho, rho45 = both(4.5f) * rho;
     const f32x2 base = mad(rho, nusq15, drho);
-    const f32x2 om = both(p.omega), om1 = both(p.one_m_omega);
     auto wmul = [&](auto I, f32x2 x) {
         constexpr int i = decltype(I)::value;
         if constexpr (EXACTW) {
@@ -152,47 +153,121 @@ __device__ __forceinline__ void bgk_pair(const StepParams<float>& p, const PairC
             return mad(both(float(L::w(i)) * sc), x, minus_zero);
         }
     };
-    auto relax = [&](auto I, f32x2 fe) {
-        constexpr int i = decltype(I)::value;
-        f32x2 o = mad(om, fe, om1 * v[i]);
-        if constexpr (SPECIAL) {
-            float a, b, c, d;
-            unpack2(o, a, b);
-            unpack2(fe, c, d);
-            if (A.fl & kEquilibrium) a = c;
-            if (B.fl & kEquilibrium) b = d;
-            if constexpr (i > 0) {
-                unpack2(v[L::opp(i)], c, d);
-                if (A.fl & kBounce) a = c;
-                if (B.fl & kBounce) b = d;
-            }
-            o = pack2(a, b);
-        }
-        out[i] = o;
-    };
     auto dirs = [&](auto I, f32x2 eu) {
-        constexpr int o = L::opp(decltype(I)::value);
         const f32x2 sym = wmul(I, mad(rho45, eu * eu, base));
         const f32x2 anti = wmul(I, rho3 * eu);
-        relax(I, sym + anti);
-        relax(std::integral_constant<int, o>{}, sym - anti);
+        put(I, sym + anti);
+        put(std::integral_constant<int, L::opp(decltype(I)::value)>{}, sym - anti);
     };
-    relax(std::integral_constant<int, 0>{}, wmul(std::integral_constant<int, 0>{}, base));
+    put(std::integral_constant<int, 0>{}, wmul(std::integral_constant<int, 0>{}, base));
     dirs(std::integral_constant<int, 1>{}, ux);
     dirs(std::integral_constant<int, 2>{}, uy);
     dirs(std::integral_constant<int, 5>{}, ux + uy);
     dirs(std::integral_constant<int, 6>{}, uy - ux);
 }
 
+// Direction i of two cells after the collision gave o: equilibrium cells take fe, solid ones what came from
+// the other side.
+template <int i, bool SPECIAL>
+__device__ __forceinline__ f32x2 pair_boundary(const PairClass& A, const PairClass& B, f32x2 o, f32x2 fe, const f32x2 (&v)[9]) {
+    if constexpr (SPECIAL) {
+        float a, b, c, d;
+        unpack2(o, a, b);
+        unpack2(fe, c, d);
+        if (A.fl & kEquilibrium) a = c;
+        if (B.fl & kEquilibrium) b = d;
+        if constexpr (i > 0) {
+            unpack2(v[D2Q9::opp(i)], c, d);
+            if (A.fl & kBounce) a = c;
+            if (B.fl & kBounce) b = d;
+        }
+        return pack2(a, b);
+    }
+    return o;
+}
+
+// bgk_collide of two D2Q9 cells at once (FP32 arithmetic on deviations v, in storage units): its operations
+// in its order, each on both lanes, so every lane's result is bgk_collide's.  A, B: the cells' classes
+// (SPECIAL; without it both are plain fluid).  No Zou-He cells.
+// minus_zero: a packed -0 the compiler cannot see through; with it a product that feeds an addition is a
+// multiply-add of the same value, which cannot be contracted into the addition.
+template <bool EXACTW, bool SPECIAL>
+__device__ __forceinline__ void bgk_pair(const StepParams<float>& p, const PairClass& A, const PairClass& B, f32x2 (&v)[9],
+                                         float sc, float isc, f32x2 minus_zero, f32x2 (&out)[9]) {
+    f32x2 rho, drho, ux, uy;
+    pair_moments<EXACTW, SPECIAL>(A, B, v, isc, rho, drho, ux, uy);
+    const f32x2 om = both(p.omega), om1 = both(p.one_m_omega);
+    pair_equilibrium<EXACTW>(rho, drho, ux, uy, sc, minus_zero, [&](auto I, f32x2 fe) {
+        constexpr int i = decltype(I)::value;
+        out[i] = pair_boundary<i, SPECIAL>(A, B, mad(om, fe, om1 * v[i]), fe, v);
+    });
+}
+
+// psi = 1 - exp(-rho) of two cells' streamed density: sc_psi_from on both lanes.
+template <bool SPECIAL>
+__device__ __forceinline__ f32x2 sc_psi_pair(const PairClass& A, const PairClass& B, const f32x2 (&v)[9], float isc) {
+    f32x2 r = v[0];
+    static_for<8>([&](auto I) { r = r + v[I + 1]; });
+    float a, b;
+    unpack2(both(1.0f) + r * both(isc), a, b);  // a power of two: the product is exact
+    if constexpr (SPECIAL) {
+        if (A.fl & kSetRho) a = A.rho;
+        if (B.fl & kSetRho) b = B.rho;
+    }
+    return pack2(1.0f - expf(-a), 1.0f - expf(-b));
+}
+
+// The Shan-Chen force (sc_force_from) and collision (sc_collide_store) of two cells: psi_at(dx, dy) gives both
+// cells' neighbours.  Every product that feeds an addition goes through minus_zero (see bgk_pair).
+template <bool EXACTW, bool SPECIAL, class PsiAt>
+__device__ __forceinline__ void sc_pair(const StepParams<float>& p, const PairClass& A, const PairClass& B, f32x2 (&v)[9],
+                                        float sc, float isc, f32x2 minus_zero, PsiAt&& psi_at, f32x2 (&out)[9]) {
+    using L = D2Q9;
+    f32x2 rho, drho, ux, uy;
+    pair_moments<EXACTW, SPECIAL>(A, B, v, isc, rho, drho, ux, uy);
+    f32x2 sx, sy;
+    static_for<8>([&](auto I) {
+        constexpr int i = I + 1, cx = L::cx(i), cy = L::cy(i);
+        const f32x2 w = mad(both(float(L::w(i))), psi_at(std::integral_constant<int, cx>{}, std::integral_constant<int, cy>{}),
+                            minus_zero);
+        if constexpr (i == 1) sx = w;
+        else if constexpr (cx == 1) sx = sx + w;
+        else if constexpr (cx == -1) sx = sx - w;
+        if constexpr (i == 2) sy = w;
+        else if constexpr (cy == 1) sy = sy + w;
+        else if constexpr (cy == -1) sy = sy - w;
+    });
+    const f32x2 g = both(-p.G) * psi_at(std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{});
+    const f32x2 orho = both(p.omega) * rho;
+    const f32x2 k = reciprocal(orho, neg(orho));
+    const f32x2 wx = ux + mad(g * sx, k, minus_zero), wy = uy + mad(g * sy, k, minus_zero);
+    float a, b, c, d, ra, rb;
+    unpack2(rho, ra, rb);  // no shift where rho <= 0
+    unpack2(ux, a, b);
+    unpack2(wx, c, d);
+    const f32x2 vx = pack2(ra > 0.0f ? c : a, rb > 0.0f ? d : b);
+    unpack2(uy, a, b);
+    unpack2(wy, c, d);
+    const f32x2 vy = pack2(ra > 0.0f ? c : a, rb > 0.0f ? d : b);
+    const f32x2 om = both(p.omega), om1 = both(p.one_m_omega);
+    pair_equilibrium<EXACTW>(rho, drho, vx, vy, sc, minus_zero, [&](auto I, f32x2 fe) {
+        constexpr int i = decltype(I)::value;
+        out[i] = pair_boundary<i, SPECIAL>(A, B, mad(om, fe, minus_zero) + mad(om1, v[i], minus_zero), fe, v);
+    });
+}
+
 // Shape of the tile kernel: source regions of up to MAXR rows of PX cells in shared memory, direction by
 // direction, HALO columns on either side of the tile's W.  MOVERS: warps that do nothing but bring the
-// next tile's region in and store the last one's tile (bulk copies; two buffers), 0: the computing warps do.
-// The steps compute the PW middle columns: T <= (PW - W) / 2.
-template <class S, int PX_, int PW_, int MAXR_, int HALO_, int WARPS_, int MOVERS_>
+// next tile's region in and store the last one's tile (two buffers), 0: the computing warps do.  BULK: they move
+// whole rows by bulk copies where rows start on 16-byte words, else pieces.
+// The steps compute the PW middle columns: D T <= (PW - W) / 2.  SC: Shan-Chen, whose step reaches D = 2 cells far
+// and keeps psi of the region besides.
+template <class S, bool SC_, int PX_, int PW_, int MAXR_, int HALO_, int WARPS_, int MOVERS_, bool BULK_>
 struct TileShape {
-    using Word = S;
+    static constexpr bool SC = SC_, BULK = BULK_;
+    static constexpr int D = SC ? 2 : 1;
     static constexpr int PX = PX_, PW = PW_, MAXR = MAXR_, HALO = HALO_, WARPS = WARPS_, MOVERS = MOVERS_;
-    static constexpr int kMaxSteps = (PW - (PX - 2 * HALO)) / 2;
+    static constexpr int kMaxSteps = (PW - (PX - 2 * HALO)) / (2 * D);
     static constexpr int NBUF = MOVERS > 0 ? 2 : 1;
     static constexpr int W = PX - 2 * HALO, THREADS = 32 * WARPS, BLOCK = THREADS + 32 * MOVERS;
     static constexpr int GUARD = 16 / (int)sizeof(S);  // words before and after a direction's region
@@ -200,13 +275,14 @@ struct TileShape {
     static constexpr int BUF = 9 * PLANE;
     static_assert((PX * sizeof(S)) % 16 == 0 && (HALO * sizeof(S)) % 16 == 0, "rows of whole 16-byte words");
     static constexpr size_t kPop = 64 + sizeof(PairClass) * kMaxClasses;
-    static constexpr size_t kCls = kPop + (size_t)NBUF * BUF * sizeof(S);
+    static constexpr size_t kPsi = kPop + (size_t)NBUF * BUF * sizeof(S);
+    static constexpr size_t kCls = kPsi + (SC ? (size_t)(MAXR * PX + 8) * sizeof(typename Codec<S>::Real) : 0);
     static constexpr size_t kClsBytes = (size_t)(MAXR * PX + 15) / 16 * 16;
     static constexpr size_t smem_bytes() { return kCls + NBUF * kClsBytes; }
 };
 
 // How a lattice's multi-step launches are cut.
-enum TileKind { kTilesNone = 0, kTilesSmall, kTilesMid, kTilesStream };
+enum TileKind { kTilesNone = 0, kTilesSmall, kTilesMid, kTilesPieces, kTilesStream, kTilesShanChen };
 struct TilePlan {
     int kind = kTilesNone;
     int h = 0;      // rows of a tile (even)
@@ -218,7 +294,7 @@ struct TileLaunch {
     int* err;
     int sms;
 };
-// The plan of a D2Q9 BGK lattice on a device of `sms` SMs (kTilesNone: single steps are faster).
+// The plan of a D2Q9 BGK or Shan-Chen lattice on a device of `sms` SMs (kTilesNone: single steps are faster).
 TilePlan plan_tiles(const lbm_desc& d, int sms);
 cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int T, cudaStream_t s);
 
@@ -241,11 +317,11 @@ __device__ __forceinline__ void bulk_store(void* dst_gmem, const void* src_smem,
                  : "memory");
 }
 
-// One tile launch: tiles of W x h cells, T (even, <= HALO) steps.  nx >= PX and ny >= h + 2 T
+// One tile launch: tiles of W x h cells, T (even, D T <= HALO) steps.  nx >= PX and ny >= h + 2 D T
 // (host-checked): every region cell wraps at most once.  CTAs walk the tiles with a stride.  A thread takes
 // two cells at a time (PX and h are even).
 // G: bytes of the pieces that regions and tiles move in, 16, 8, 4 or (16-bit words) 2: every row of the
-// lattice starts on a multiple of it (16 with movers).
+// lattice starts on a multiple of it.
 template <class S, bool ABS, class Sh, int G>
 __global__ void __launch_bounds__(Sh::BLOCK, 1)
     k_step_tiles(const __grid_constant__ StepParams<typename Codec<S>::Real> p, int h, int T, int tiles_x, int tiles,
@@ -262,11 +338,13 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
     S* const pops = reinterpret_cast<S*>(smem + Sh::kPop) + Sh::GUARD;
     const int tid = (int)threadIdx.x;
     const int nx = p.nx, ny = p.ny;
-    const int rows = h + 2 * T;  // of the source region
+    const int depth = Sh::D * T, rows = h + 2 * depth;  // rows of the source region
     const uint32_t N = (uint32_t)p.N;  // 9 N <= 2^32 (host-checked)
     const int stride = (int)gridDim.x;
     constexpr int GW = G / (int)sizeof(S);  // cells of a piece
-    static_assert(GW >= 1 && GW * (int)sizeof(S) == G && (!kMove || G == 16), "pieces of whole words");
+    static_assert(GW >= 1 && GW * (int)sizeof(S) == G, "pieces of whole words");
+    constexpr bool SC = Sh::SC, kBulk = kMove && Sh::BULK && G == 16;
+    static_assert(!SC || kPacked, "Shan-Chen tiles: packed FP32 arithmetic");
     using Piece = std::conditional_t<G == 16, uint4, std::conditional_t<G == 8, uint2, std::conditional_t<G == 4, uint32_t, uint16_t>>>;
 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -274,7 +352,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
     if constexpr (kMove) {
         if (tid == 0) {
             for (int b = 0; b < NBUF; ++b) {
-                mbar_init(&full[b], 1);
+                mbar_init(&full[b], kBulk ? 1 : 32 * Sh::MOVERS);
                 mbar_init(&done[b], 1);
             }
             mbar_init_fence();
@@ -298,7 +376,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
     // from global memory, and with their marks to shared memory (returns the marks among them).
     constexpr int kClsWords = (Sh::MAXR * (PX / 4) + THREADS - 1) / THREADS;
     auto get_classes = [&](int n, uint32_t (&c)[kClsWords]) {
-        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - T;
+        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - depth;
         static_for<kClsWords>([&](auto J) {
             const int j = tid + decltype(J)::value * THREADS;
             c[J] = 0;
@@ -325,76 +403,18 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
     };
     const bool classes = has_mask || mark(0u) != 0;  // some cell of the lattice may not be plain fluid
 
-    if constexpr (kMove) {
-        if (tid >= THREADS) {
-            constexpr int MT = 32 * Sh::MOVERS;
-            const int m = tid - THREADS;
-            auto move_in = [&](int n, int b) {
-                const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - T;
-                const S* __restrict__ const fin = static_cast<const S*>(p.fin);
-                const int a = x0 < 0 ? x0 + nx : x0, len = nx - a < PX ? nx - a : PX;  // before the wrap in x
-                if (m == 0) mbar_arrive_expect_tx(&full[b], (uint32_t)(Q * rows * PX * (int)sizeof(S)));
-                for (int j = m; j < Q * rows; j += MT) {
-                    const int ly = j / Q, i = j - ly * Q;
-                    int y = y0 + ly;
-                    y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
-                    const S* const row = fin + ((size_t)i * N + (size_t)((uint32_t)y * (uint32_t)nx));
-                    S* const dst = pops + b * Sh::BUF + i * PLANE + ly * PX;
-                    bulk_load(dst, row + a, (uint32_t)(len * (int)sizeof(S)), &full[b]);
-                    if (len < PX) bulk_load(dst + len, row, (uint32_t)((PX - len) * (int)sizeof(S)), &full[b]);
-                }
-            };
-            int n = (int)blockIdx.x;
-            for (int b = 0; b < NBUF; ++b)
-                if (n + b * stride < tiles) move_in(n + b * stride, b);
-            for (int turn = 0; n < tiles; ++turn, n += stride) {
-                const int b = turn & 1;
-                const bool ok = mbar_wait_bounded(&done[b], (uint32_t)((turn >> 1) & 1));
-                if (!ok) {
-                    atomicExch(err, kRowPipeTimeout);
-                    break;
-                }
-                const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W, y0 = ty * h;
-                const int w = nx - x0 < W ? nx - x0 : W, hh = ny - y0 < h ? ny - y0 : h;
-                S* const fout = static_cast<S*>(p.fout);
-                for (int j = m; j < Q * hh; j += MT) {
-                    const int r = j / Q, i = j - r * Q;
-                    bulk_store(fout + ((size_t)i * N + (size_t)((uint32_t)(y0 + r) * (uint32_t)nx + (uint32_t)x0)),
-                               pops + b * Sh::BUF + i * PLANE + (r + T) * PX + HALO, (uint32_t)(w * (int)sizeof(S)));
-                }
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                if (n + NBUF * stride < tiles) {
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    asm volatile("bar.sync 2, %0;" ::"n"(MT) : "memory");  // every mover's stores have read the buffer
-                    move_in(n + NBUF * stride, b);
-                }
-            }
-            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-            return;
-        }
-    }
-    auto barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); };
-    auto any = [](bool v) {
-        int r;
-        asm volatile(
-            "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-            : "=r"(r)
-            : "r"((unsigned)v), "n"(THREADS)
-            : "memory");
-        return r != 0;
-    };
-
-    // The source region of tile n: f_i of cell (x0 + lx, y0 + ly) to [i][ly PX + lx].
-    auto move_in = [&](int n) {
-        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - T;
+    // The source region of tile n into buffer b, f_i of cell (x0 + lx, y0 + ly) to [i][ly PX + lx], and tile n
+    // out of buffer b, in pieces, by `count` threads.
+    auto pieces_in = [&](int n, int b, int who, int count) {
+        const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - depth;
         const char* const fin = static_cast<const char*>(p.fin);
-        for (int j = tid; j < rows * (PX / GW); j += THREADS) {
+        for (int j = who; j < rows * (PX / GW); j += count) {
             const int ly = j / (PX / GW), lx = (j - ly * (PX / GW)) * GW;
             int x = x0 + lx, y = y0 + ly;
             x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
             y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
             const uint32_t off = ((uint32_t)y * (uint32_t)nx + (uint32_t)x) * (uint32_t)sizeof(S);
-            S* const dst = pops + ly * PX + lx;
+            S* const dst = pops + b * Sh::BUF + ly * PX + lx;
             static_for<Q>([&](auto I) {
                 constexpr int i = I;
                 const char* const base = fin + (size_t)i * N * sizeof(S);
@@ -410,12 +430,11 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
             });
         }
     };
-    // Tile n out.
-    auto move_out = [&](int n) {
+    auto pieces_out = [&](int n, int b, int who, int count) {
         const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W, y0 = ty * h;
         char* const fout = static_cast<char*>(p.fout);
-        const S* const buf = pops + T * PX + HALO;
-        for (int j = tid; j < h * (W / GW); j += THREADS) {
+        const S* const buf = pops + b * Sh::BUF + depth * PX + HALO;
+        for (int j = who; j < h * (W / GW); j += count) {
             const int ly = j / (W / GW), lx = (j - ly * (W / GW)) * GW;
             const int x = x0 + lx, y = y0 + ly;
             if (x >= nx || y >= ny) continue;
@@ -428,6 +447,83 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
             });
         }
     };
+    // barrier of one group of warps (1: computing, 2: moving) and its vote
+    auto vote = [](int id, int count, bool v) {
+        int r;
+        asm volatile(
+            "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+            : "=r"(r)
+            : "r"((unsigned)v), "r"(id), "r"(count)
+            : "memory");
+        return r != 0;
+    };
+
+    if constexpr (kMove) {
+        if (tid >= THREADS) {
+            constexpr int MT = 32 * Sh::MOVERS;
+            const int m = tid - THREADS;
+            auto move_in = [&](int n, int b) {
+                if constexpr (!kBulk) {
+                    pieces_in(n, b, m, MT);
+                    if constexpr (G >= 4)  // arrives when this thread's copies have landed
+                        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(&full[b])) : "memory");
+                    else
+                        mbar_arrive(&full[b]);
+                } else {
+                    const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W - HALO, y0 = ty * h - depth;
+                    const S* __restrict__ const fin = static_cast<const S*>(p.fin);
+                    const int a = x0 < 0 ? x0 + nx : x0, len = nx - a < PX ? nx - a : PX;  // before the wrap in x
+                    if (m == 0) mbar_arrive_expect_tx(&full[b], (uint32_t)(Q * rows * PX * (int)sizeof(S)));
+                    for (int j = m; j < Q * rows; j += MT) {
+                        const int ly = j / Q, i = j - ly * Q;
+                        int y = y0 + ly;
+                        y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+                        const S* const row = fin + ((size_t)i * N + (size_t)((uint32_t)y * (uint32_t)nx));
+                        S* const dst = pops + b * Sh::BUF + i * PLANE + ly * PX;
+                        bulk_load(dst, row + a, (uint32_t)(len * (int)sizeof(S)), &full[b]);
+                        if (len < PX) bulk_load(dst + len, row, (uint32_t)((PX - len) * (int)sizeof(S)), &full[b]);
+                    }
+                }
+            };
+            auto move_out = [&](int n, int b) {
+                if constexpr (!kBulk) {
+                    pieces_out(n, b, m, MT);
+                } else {
+                    const int ty = n / tiles_x, x0 = (n - ty * tiles_x) * W, y0 = ty * h;
+                    const int w = nx - x0 < W ? nx - x0 : W, hh = ny - y0 < h ? ny - y0 : h;
+                    S* const fout = static_cast<S*>(p.fout);
+                    for (int j = m; j < Q * hh; j += MT) {
+                        const int r = j / Q, i = j - r * Q;
+                        bulk_store(fout + ((size_t)i * N + (size_t)((uint32_t)(y0 + r) * (uint32_t)nx + (uint32_t)x0)),
+                                   pops + b * Sh::BUF + i * PLANE + (r + depth) * PX + HALO, (uint32_t)(w * (int)sizeof(S)));
+                    }
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            };
+            int n = (int)blockIdx.x;
+            for (int b = 0; b < NBUF; ++b)
+                if (n + b * stride < tiles) move_in(n + b * stride, b);
+            for (int turn = 0; n < tiles; ++turn, n += stride) {
+                const int b = turn & 1;
+                const bool ok = mbar_wait_bounded(&done[b], (uint32_t)((turn >> 1) & 1));
+                if (vote(2, MT, !ok)) {
+                    if (!ok) atomicExch(err, kRowPipeTimeout);
+                    break;
+                }
+                move_out(n, b);
+                if (n + NBUF * stride < tiles) {
+                    if constexpr (kBulk) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    vote(2, MT, false);  // every mover has read its part of the buffer
+                    move_in(n + NBUF * stride, b);
+                }
+            }
+            if constexpr (kBulk) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return;
+        }
+    }
+    auto barrier = [] { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); };
+    auto any = [&](bool v) { return vote(1, THREADS, v); };
 
     R sc, isc;
     storage_scale<S>(p, sc, isc);
@@ -447,16 +543,15 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
     for (int turn = 0, n = (int)blockIdx.x; n < tiles; ++turn, n += stride) {
         const int b = NBUF == 2 ? turn & 1 : 0;
         const int ty = n / tiles_x, tx = n - ty * tiles_x;
-        const int x0 = tx * W - HALO, y0 = ty * h - T;
+        const int x0 = tx * W - HALO, y0 = ty * h - depth;
         S* const pop = pops + b * Sh::BUF;
-        if constexpr (!kMove) move_in(n);
+        if constexpr (!kMove) pieces_in(n, 0, tid, THREADS);
         const uint8_t* const cls_s = smem + Sh::kCls + b * Sh::kClsBytes;
         uint32_t kind = 0;  // marks among the region's cells
         if constexpr (kMove) {
-            if (!mbar_wait_bounded(&full[b], (uint32_t)((turn >> 1) & 1))) {
-                atomicExch(err, kRowPipeTimeout);
-                return;
-            }
+            const bool ok = mbar_wait_bounded(&full[b], (uint32_t)((turn >> 1) & 1));
+            if (!ok) atomicExch(err, kRowPipeTimeout);
+            if (any(!ok)) return;
         } else {
             if (classes) {
                 get_classes(n, next_cls);
@@ -484,10 +579,11 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
             // meet in a bank) half the rows apart
             constexpr bool adj = !around || k16;
             constexpr int PW = Sh::PW;
-            const int half = (rows / 2 - t) * PX;
-            const int count = (rows / 2 - t) * PW, second = adj ? 1 : half;  // pairs of cells
-            const int first = t * PX;
-            if constexpr (SPECIAL) {
+            const int edge = Sh::D * t;  // the outermost rows that are not computed
+            const int half = (rows / 2 - edge) * PX;
+            const int count = (rows / 2 - edge) * PW, second = adj ? 1 : half;  // pairs of cells
+            const int first = edge * PX;
+            if constexpr (SPECIAL && !SC) {
                 // A zero-gradient cell's c_x = -1 populations are f_i(x, y - c_iy) of its own column, which
                 // the cell to its left reads and overwrites.  They are copied to where the cell itself
                 // reads, which no other cell touches in this step.
@@ -523,16 +619,21 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                     }
                 }
             }
-#pragma unroll 1
-            for (int j = tid; j < count; j += THREADS) {
-                int k = first + (adj ? 2 * j : j);
+            auto value = [&](S w, auto I) -> R {
+                if constexpr (ABS)
+                    return R(w);
+                else
+                    return Codec<S>::raw(w, R(L::w(decltype(I)::value)));
+            };
+            auto pair_of = [&](int j, int from) {  // first cell of pair j of the rows from `from` on
+                int k = from + (adj ? 2 * j : j);
                 if constexpr (PW < PX) {
                     constexpr int PR = adj ? PW / 2 : PW;  // pairs of a row
                     k += (j / PR) * (PX - PW) + (PX - PW) / 2;
                 }
-                S* const c = pop + k;
-                S* const d = c + second;
-                S wA[Q], wB[Q];
+                return k;
+            };
+            auto load_pair = [&](const S* c, const S* d, S(&wA)[Q], S(&wB)[Q]) {
                 static_for<Q>([&](auto I) {
                     constexpr int i = I, o = around ? i * PLANE - (L::cy(i) * PX + L::cx(i)) : L::opp(i) * PLANE;
                     if constexpr (adj && (!around || L::cx(i) == 0)) {
@@ -544,17 +645,55 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                         wB[i] = d[o];
                     }
                 });
+            };
+            auto pack_pair = [&](const S(&wA)[Q], const S(&wB)[Q], f32x2(&v)[Q]) {
+                static_for<Q>([&](auto I) {
+                    constexpr int i = I;
+                    if constexpr (k16)
+                        v[i] = pack2(value(wA[i], I), value(wB[i], I));
+                    else if constexpr (kPacked)
+                        v[i] = pack2(wA[i], wB[i]) - both(float(L::w(i)));
+                });
+            };
+            [[maybe_unused]] R* const psi = reinterpret_cast<R*>(smem + Sh::kPsi) + 4;
+            if constexpr (SC) {
+                // psi of the streamed densities, one cell further out than what is collided
+                const int rim = edge - 1, apart = (rows / 2 - rim) * PX, away = adj ? 1 : apart;
+#pragma unroll 1
+                for (int j = tid; j < (rows / 2 - rim) * PW; j += THREADS) {
+                    const int k = pair_of(j, rim * PX);
+                    S wA[Q], wB[Q];
+                    f32x2 v[Q];
+                    load_pair(pop + k, pop + k + away, wA, wB);
+                    pack_pair(wA, wB, v);
+                    PairClass A{}, B{};
+                    if constexpr (SPECIAL) {
+                        A = table[cls_s[k] & kMarkClass];
+                        B = table[cls_s[k + away] & kMarkClass];
+                    }
+                    float a, b2;
+                    unpack2(sc_psi_pair<SPECIAL>(A, B, v, isc), a, b2);
+                    if constexpr (adj) {
+                        *reinterpret_cast<float2*>(psi + k) = float2{a, b2};
+                    } else {
+                        psi[k] = a;
+                        psi[k + away] = b2;
+                    }
+                }
+                barrier();
+            }
+#pragma unroll 1
+            for (int j = tid; j < count; j += THREADS) {
+                const int k = pair_of(j, first);
+                S* const c = pop + k;
+                S* const d = c + second;
+                S wA[Q], wB[Q];
+                load_pair(c, d, wA, wB);
                 uint32_t mA = 0, mB = 0;
                 if constexpr (SPECIAL) {
                     mA = cls_s[k];
                     mB = cls_s[k + second];
                 }
-                auto value = [&](S w, auto I) -> R {
-                    if constexpr (ABS)
-                        return R(w);
-                    else
-                        return Codec<S>::raw(w, R(L::w(decltype(I)::value)));
-                };
                 R oA[Q], oB[Q];  // stored values: collided deviations for the 16-bit codecs, populations else
                 auto scalar = [&](const S(&w)[Q], uint32_t m, R(&o)[Q]) {
                     R v[Q], out[Q];
@@ -572,19 +711,26 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                 if constexpr (kPacked) {
                     auto packed = [&](auto Sp) {
                         f32x2 v[Q], out[Q];
-                        static_for<Q>([&](auto I) {
-                            constexpr int i = I;
-                            if constexpr (k16)
-                                v[i] = pack2(value(wA[i], I), value(wB[i], I));
-                            else
-                                v[i] = pack2(wA[i], wB[i]) - both(float(L::w(i)));
-                        });
+                        pack_pair(wA, wB, v);
                         PairClass A{}, B{};
                         if constexpr (decltype(Sp)::value) {
                             A = table[mA & kMarkClass];
                             B = table[mB & kMarkClass];
                         }
-                        bgk_pair<kExactWeights<S>, decltype(Sp)::value>(p, A, B, v, sc, isc, both(minus_zero), out);
+                        if constexpr (SC) {
+                            auto psi_at = [&](auto DX, auto DY) {
+                                constexpr int dx = decltype(DX)::value, o = decltype(DY)::value * PX + dx;
+                                if constexpr (adj && dx == 0) {
+                                    const float2 q = *reinterpret_cast<const float2*>(psi + k + o);
+                                    return pack2(q.x, q.y);
+                                } else {
+                                    return pack2(psi[k + o], psi[k + second + o]);
+                                }
+                            };
+                            sc_pair<kExactWeights<S>, decltype(Sp)::value>(p, A, B, v, sc, isc, both(minus_zero), psi_at, out);
+                        } else {
+                            bgk_pair<kExactWeights<S>, decltype(Sp)::value>(p, A, B, v, sc, isc, both(minus_zero), out);
+                        }
                         static_for<Q>([&](auto I) {
                             constexpr int i = I;
                             // F32: the stored word w + d
@@ -595,11 +741,11 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                         packed(std::false_type{});
                     } else if (!__any_sync(__activemask(), ((mA | mB) & kMarkFlags) != 0u)) {
                         packed(std::false_type{});
-                    } else if (kind & kMarkZouHe) {
+                    } else if (SC || !(kind & kMarkZouHe)) {
+                        packed(std::true_type{});
+                    } else {
                         scalar(wA, mA, oA);
                         scalar(wB, mB, oB);
-                    } else {
-                        packed(std::true_type{});
                     }
                 } else {
                     scalar(wA, mA, oA);
@@ -632,7 +778,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                     });
                 }
             }
-            if (kMove && !around && t == T) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (kBulk && !around && t == T) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             barrier();
         };
         auto steps = [&](auto Special) {
@@ -650,7 +796,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
             if (tid == 0) mbar_arrive(&done[b]);
             if (classes && n + stride < tiles) seen = put_classes(next_cls, b ^ 1);
         } else {
-            move_out(n);
+            pieces_out(n, 0, tid, THREADS);
             if (n + stride < tiles) barrier();
         }
     }

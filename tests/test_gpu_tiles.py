@@ -1,4 +1,4 @@
-"""Several steps per launch on overlapped tiles (csrc/tiles.cuh): a D2Q9 BGK lattice whose kernel family is
+"""Several steps per launch on overlapped tiles (csrc/tiles.cuh): a D2Q9 lattice whose kernel family is
 left to the engine gives the same populations, macros and residual as one stepped by the plain kernel, bit
 for bit: every storage and arithmetic, each tile shape, remainders of tiles and of steps, all boundary
 classes."""
@@ -77,13 +77,44 @@ def test_tiles_equal_plain_steps_in_absolute_arithmetic(kind, nx, ny, storage):
     same(kind, nx, ny, storage, ABS, (3, 20))
 
 
-@pytest.mark.parametrize("kind,nx,ny", [
-    (1, 1200, 1000),          # streamed tiles
-    ("periodic", 1068, 1067), # a short last tile in x and y
-    ("lid", 1501, 1201),      # one region at a time: rows that start anywhere
+@pytest.mark.parametrize("storage,kind,nx,ny", [
+    (lb.F32, "lid", 1024, 512),        # in L2, two waves: moved in pieces
+    (lb.F32, 1, 1200, 1000),           # streamed by bulk copies
+    (lb.F32, "periodic", 1068, 1067),  # a short last tile in x and y
+    (lb.F32, 1, 1501, 1201),           # rows that start anywhere: moved in pieces
+    (lb.F64, 1, 1030, 1000),           # streamed by bulk copies
 ])
-def test_large_fp32_lattices(kind, nx, ny):
-    same(kind, nx, ny, lb.F32, DEV, (7, 12))
+def test_many_tiles_per_cta(storage, kind, nx, ny):
+    same(kind, nx, ny, storage, DEV, (7, 12))
+
+
+@pytest.mark.parametrize("storage", [lb.F32, lb.F16S, lb.BF16S])
+@pytest.mark.parametrize("walls", [False, True])
+@pytest.mark.parametrize("nx,ny", [
+    (80, 10),     # the smallest
+    (133, 97),    # remainders; rows that start anywhere (FP32; 16-bit words step singly)
+    (136, 61),
+    (520, 500),   # one wave of full tiles
+    (1000, 900),  # several tiles a CTA
+])
+def test_shan_chen_tiles_equal_the_two_passes(nx, ny, walls, storage):
+    d = lb.make_desc(lb.D2Q9, lb.SHANCHEN, storage, (nx, ny), omega=1.1, sc_G=-5.0)
+    m = None
+    if walls:  # solid rows, a forced-density equilibrium block, a row of forced velocity
+        m = np.zeros((nx, ny), np.uint8)
+        m[:, 0] = m[:, -1] = 1
+        m[nx // 3:nx // 3 + 5, ny // 2:ny // 2 + 4] = 2
+        m[:, ny // 4] = 3
+        solid = lb.BOUNCE | lb.SET_RHO | lb.SET_UX | lb.SET_UY
+        lb.set_classes(d, [(0, 1.0, 0.0, 0.0, 0.0), (solid, 0.3, 0.0, 0.0, 0.0),
+                           (lb.EQUILIBRIUM | lb.SET_RHO, 0.8, 0.0, 0.0, 0.0), (lb.SET_UX, 1.0, 0.01, 0.0, 0.0)])
+    _, _, _, w, _ = lb.velocities(lb.D2Q9)
+    rho = 0.693 + np.random.default_rng(nx + ny).uniform(-0.05, 0.05, nx * ny)
+    F = (w[:, None] * rho[None, :]).astype(np.float32).ravel()
+    a = run(d, m, F, lb.KERNEL_AUTO, (1, 2, 3, 6, 9))
+    b = run(d, m, F, lb.KERNEL_PLAIN, (1, 2, 3, 6, 9))
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y, equal_nan=True)
 
 
 def test_nearest_rounding_and_cell_offset():
