@@ -867,11 +867,16 @@ static int check_device(int dev) {
         return set_error(LBM_ERR_NO_DEVICE, "no CUDA device visible");
     }
     if (dev < 0 || dev >= n) return set_error(LBM_ERR_INVALID, "device ordinal out of range");
-    cudaDeviceProp prop;
-    LBM_CK(cudaGetDeviceProperties(&prop, dev));
-    if (prop.major != 10 || prop.minor != 0)
+    // (single attributes: cudaGetDeviceProperties asks the driver for all of them, 3 to 40 ms a call)
+    int major = 0, minor = 0;
+    LBM_CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+    LBM_CK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
+    if (major != 10 || minor != 0) {
+        cudaDeviceProp prop;
+        LBM_CK(cudaGetDeviceProperties(&prop, dev));
         return set_error(LBM_ERR_NO_DEVICE, std::string("liblbm_b200 is built for sm_100a (B200); device is ") +
                                                 prop.name);
+    }
     return LBM_OK;
 }
 
