@@ -13,12 +13,14 @@ namespace lbm {
 // answers, but take some 20 issue slots each: they win where the populations stream from HBM (4096^2 FP32 113 us a
 // step against 126 in pieces, 2048 x 1024 19.2 against 20.5), pieces where they stay in L2 (1024^2 10.6 against
 // 11.2) and for Shan-Chen's two steps a launch (1024^2 15.1 against 17.5).
+// Mid: 16 warps, whose pairs a step make three full turns with 113 registers a thread (24 warps with 80: two turns, and
+// slower: FP16S 1000 x 300 4.28 -> 4.03, FP32 256^2 1.74 -> 1.61, 1024 x 256 cavity 3.38 -> 3.27).
 template <class S>
 constexpr int kMidHalo = sizeof(S) == 2 ? 8 : 4;
 template <class S>
 using SmallShape = TileShape<S, false, 32, 32, 24, 8, 12, 0, false>;
 template <class S>
-using MidShape = TileShape<S, false, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 8 ? 40 : 44, kMidHalo<S>, sizeof(S) == 8 ? 16 : 24, 0, false>;
+using MidShape = TileShape<S, false, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 8 ? 40 : 44, kMidHalo<S>, 16, 0, false>;
 template <class S, bool BULK>
 using StreamShape =
     TileShape<S, false, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 8 ? 20 : 42, kMidHalo<S>, sizeof(S) == 8 ? 12 : 20, 4, BULK>;
@@ -105,8 +107,8 @@ cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan&
 // When tiles are faster than single steps (measured on B200, lid cavities, us per step, single -> tiles).
 // - BGK lattices that one wave of CTAs covers: a launch of T steps then costs about 2 us of launch and drain, 2 us of
 //   moves and T short steps.  Small tiles first, for more CTAs: 96^2 FP32 1.4 -> 0.9, 128^2 1.8 -> 1.0, 192^2
-//   (16-row tiles, 4 steps) 3.5 -> 1.5; then 64-column tiles: 256^2 4.7 -> 1.8, 512^2 4.6 -> 3.5, 1000 x 300 5.0 ->
-//   3.7 (FP16S 512^2 6.2 -> 4.0, 1000 x 300 5.0 -> 4.3).  FP64 collisions take twice as long, so only up to
+//   (16-row tiles, 4 steps) 3.5 -> 1.5; then 64-column tiles: 256^2 4.7 -> 1.6, 512^2 4.6 -> 3.3, 1000 x 300 5.0 ->
+//   3.7 (FP16S 512^2 6.2 -> 4.0, 1000 x 300 5.0 -> 4.0).  FP64 collisions take twice as long, so only up to
 //   14 rows: 256^2 4.1 -> 2.7, 384^2 (16 rows) 4.3 -> 4.2, 512^2 5.3 -> 6.3.
 // - FP32 BGK in L2, several waves: a wave of h-row tiles takes 2.3 (h + 6) / 36 us, a launch 1.4, a single step 1.5
 //   and its cells at 107 G/s, which decides (1024 x 512 6.6 -> 6.2, 1024^2 11.2 -> 10.6; 1500 x 451 8.0 -> 8.7 stays

@@ -281,6 +281,15 @@ struct TileShape {
     static constexpr size_t smem_bytes() { return kCls + NBUF * kClsBytes; }
 };
 
+// bgk_collide out of line, for the rare cells that the packed collision leaves (Zou-He): keeps the loop short.
+template <bool EXACTW>
+__device__ __noinline__ void tile_collide(const StepParams<float>& p, int cls, float* v, float sc, float isc) {
+    float w[9], out[9];
+    static_for<9>([&](auto I) { w[I] = v[I]; });
+    bgk_collide<D2Q9, false, EXACTW>(p, cls, p.cls.flags[cls], w, sc, isc, out);
+    static_for<9>([&](auto I) { v[I] = out[I]; });
+}
+
 // How a lattice's multi-step launches are cut.
 enum TileKind { kTilesNone = 0, kTilesSmall, kTilesMid, kTilesPieces, kTilesStream, kTilesShanChen };
 struct TilePlan {
@@ -699,7 +708,12 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                     R v[Q], out[Q];
                     const int cls = (int)(m & kMarkClass);
                     static_for<Q>([&](auto I) { v[I] = value(w[I], I); });
-                    bgk_collide<L, ABS, kExactWeights<S>>(p, cls, SPECIAL ? p.cls.flags[cls] : 0u, v, sc, isc, out);
+                    if constexpr (kPacked) {
+                        tile_collide<kExactWeights<S>>(p, cls, v, sc, isc);
+                        static_for<Q>([&](auto I) { out[I] = v[I]; });
+                    } else {
+                        bgk_collide<L, ABS, kExactWeights<S>>(p, cls, SPECIAL ? p.cls.flags[cls] : 0u, v, sc, isc, out);
+                    }
                     static_for<Q>([&](auto I) {
                         constexpr int i = I;
                         if constexpr (k16 || ABS)
