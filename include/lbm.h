@@ -148,8 +148,9 @@ int         lbm_q(int lattice);                          /* 9 or 27 */
 int         lbm_velocities(int lattice, int32_t* cx, int32_t* cy, int32_t* cz, double* w, int32_t* opp);
 
 /* ---- single lattice ---------------------------------------------------------------------
- * lbm_create: validates the descriptor, allocates two population buffers (ping-pong) plus the mask
- * on the device, and sets every population to feq(rho=1, u=0) of each cell's class values.       */
+ * lbm_create: validates the descriptor, allocates two population buffers (ping-pong), the mask and, for
+ * D2Q9 lattices that one wave of tiles covers, what the tiles exchange (at most 20 MB) on the device,
+ * and sets every population to feq(rho=1, u=0) of each cell's class values.                          */
 int  lbm_create(const lbm_desc* d, lbm_ctx** out);
 void lbm_destroy(lbm_ctx* c);
 /* Populations in the reference layout [nx,ny(,nz),Q].  src/dst: host or device pointer. */
@@ -225,8 +226,9 @@ int   lbm_get_block(const lbm_ctx* c);
  * the cluster's shared memory for up to 4096 steps of one launch, one cluster barrier per step, for
  * lattices too small to fill the GPU (a step is then launch-bound); lbm_step_planes and lone steps
  * inside CUDA graphs take PLAIN.  AUTO (default): the autotuner times the eligible ones; besides, runs of
- * three and more steps of a D2Q9 BGK lattice advance several steps per launch, on overlapped tiles in
- * shared memory, where that is faster (lattices that one wave of CTAs covers, and FP32 ones beyond L2).
+ * three and more steps of a D2Q9 BGK or Shan-Chen lattice advance several steps per launch, on
+ * overlapped tiles in shared memory, where that is faster (BGK lattices that one wave of CTAs covers,
+ * which stay there for the whole run; FP32 and FP64 ones beyond L2; most Shan-Chen ones).
  * All give bit-identical results.                                                                   */
 enum lbm_kernel { LBM_KERNEL_AUTO = 0, LBM_KERNEL_PLAIN = 1, LBM_KERNEL_ROWS = 2, LBM_KERNEL_CLUSTER = 3 };
 int   lbm_set_kernel(lbm_ctx* c, int kind);

@@ -812,7 +812,7 @@ int lbm_batch_create(const lbm_desc* descs, int n, lbm_batch** out) {
     b->descs.assign(descs, descs + n);
     for (int k = 0; k < n; ++k) {
         lbm_ctx* m = nullptr;
-        int rc = lbm_create(&descs[k], &m);
+        int rc = create_lattice(&descs[k], &m, true);
         if (rc) {
             batch_free(b);
             return rc;

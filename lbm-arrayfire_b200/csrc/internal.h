@@ -28,6 +28,8 @@ int validate_desc(const lbm_desc* d);
 
 // Number of cells, populations per cell, bytes per stored population.
 long long desc_cells(const lbm_desc* d);
+// lbm_create; member: of an ensemble, without what only lbm_step of the lattice alone uses.
+int create_lattice(const lbm_desc* d, lbm_ctx** out, bool member);
 int desc_q(const lbm_desc* d);
 int storage_bytes(int storage);
 double default_scale(int storage);

@@ -153,6 +153,7 @@ struct lbm_ctx {
     int rows_rpg = 1;              // its rows per group (segmented rows: the segment width)
     long long scw_target = 0;      // Shan-Chen window kernel: resident CTAs of the device (0: not queried)
     int* err = nullptr;            // device error word of the row pipeline
+    TileExchange tile_ex;          // what its tiles exchange
     unsigned* tick = nullptr;      // the rounding's step counter pair (step_rounding)
     WaitLimits waits = kProductionWaits;  // the row pipeline's wait limits for the next launch
     bool stall_armed = false;      // lbm_test_stall_next_step: the next step launches with `stall`
@@ -667,11 +668,34 @@ static cudaError_t launch_tiles(lbm_ctx* c, int from, cudaStream_t s, int T) {
     l.pf = c->pf;
     l.pd = c->pd;
     l.err = c->err;
+    l.ex = c->tile_ex;
     l.sms = c->sms;
     l.pf.fin = l.pd.fin = c->f[from];
     l.pf.fout = l.pd.fout = c->f[from ^ 1];
     l.pf.parity = l.pd.parity = from;
     return launch_tiles(c->d, l, c->tiles, T, s);
+}
+
+// The plan, and whether its tiles can run in rounds: what they exchange is allocated with the lattice, or at the first
+// run that is long enough (members of an ensemble, which the ensemble steps).  Not in a capture, nor where memory is
+// out: then one launch a round.
+static bool tiles_ready(lbm_ctx* c) {
+    if (!c->sms && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->d.device) != cudaSuccess) return false;
+    c->tiles = plan_tiles(c->d, c->sms);
+    TileExchange& e = c->tile_ex;
+    if (e.records) return true;
+    e = tile_exchange(c->d, c->tiles);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!e.bytes || cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+    const size_t all = e.bytes + sizeof(unsigned) * c->sms;
+    if (cudaMalloc(&e.records, all) != cudaSuccess || cudaMemsetAsync(e.records, 0, all, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(e.records);
+        e = TileExchange{};
+        return false;
+    }
+    e.rounds = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(e.records) + e.bytes);
+    return true;
 }
 
 static std::mutex g_tune_mu;
@@ -840,6 +864,7 @@ static void destroy_ctx(lbm_ctx* c) {
     cudaFree(c->sums_out);
     cudaFree(c->err);
     cudaFree(c->tick);
+    cudaFree(c->tile_ex.records);
     if (c->e0) cudaEventDestroy(c->e0);
     if (c->e1) cudaEventDestroy(c->e1);
     if (c->own) cudaStreamDestroy(c->own);
@@ -880,11 +905,7 @@ static int check_device(int dev) {
     return LBM_OK;
 }
 
-}  // namespace lbm
-
-extern "C" {
-
-int lbm_create(const lbm_desc* d, lbm_ctx** out) {
+int create_lattice(const lbm_desc* d, lbm_ctx** out, bool member) {
     if (!out) return set_error(LBM_ERR_INVALID, "out is NULL");
     *out = nullptr;
     int rc = validate_desc(d);
@@ -935,6 +956,7 @@ int lbm_create(const lbm_desc* d, lbm_ctx** out) {
     c->mrt2 = mrt2_applies(c->d);
     c->pf = make_params<float>(c);
     c->pd = make_params<double>(c);
+    if (!member && tiles_apply(c)) tiles_ready(c);
     rc = lbm_init_equilibrium(c, nullptr, nullptr);
     if (rc) {
         destroy_ctx(c);
@@ -943,6 +965,12 @@ int lbm_create(const lbm_desc* d, lbm_ctx** out) {
     *out = c;
     return LBM_OK;
 }
+
+}  // namespace lbm
+
+extern "C" {
+
+int lbm_create(const lbm_desc* d, lbm_ctx** out) { return create_lattice(d, out, false); }
 
 void lbm_destroy(lbm_ctx* c) { destroy_ctx(c); }
 
@@ -1068,11 +1096,10 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
     LBM_CK(cudaEventRecord(c->e0, c->stream));
     long long n = nsteps;
     if (tiles_apply(c)) {
-        if (!c->sms) LBM_CK(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->d.device));
-        c->tiles = plan_tiles(c->d, c->sms);
+        const int most = tiles_ready(c) ? tile_launch_steps(c->tiles) : c->tiles.steps;
         // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
         while (c->tiles.kind != kTilesNone && n > 2) {
-            const int k = (int)std::min<long long>((n - 1) / 2 * 2, c->tiles.steps);
+            const int k = (int)std::min<long long>((n - 1) / 2 * 2, most);
             LBM_CK(launch_tiles(c, c->cur, c->stream, k));
             c->cur ^= 1;
             n -= k;
@@ -1127,6 +1154,9 @@ int lbm_sync(lbm_ctx* c) {
     LBM_CK(cudaMemcpy(&err, c->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) {
         LBM_CK(cudaMemset(c->err, 0, sizeof(int)));
+        if (c->tile_ex.records) {  // tiles that gave up are behind the others
+            LBM_CK(cudaMemset(c->tile_ex.records, 0, c->tile_ex.bytes + sizeof(unsigned) * c->sms));
+        }
         return set_error(LBM_ERR_TIMEOUT, "a row-pipeline wait on a shared-memory stage gave up; results are invalid");
     }
     return LBM_OK;

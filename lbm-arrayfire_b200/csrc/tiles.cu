@@ -28,18 +28,30 @@ template <class S>
 using ShanChenShape = TileShape<S, true, 64 + 2 * kMidHalo<S>, 72, sizeof(S) == 2 ? 44 : 40, kMidHalo<S>, 20, 4, false>;
 
 template <class S, bool ABS, class Sh, int G>
-static cudaError_t launch_one(const StepParams<typename Codec<S>::Real>& p, const TileLaunch& l, const TilePlan& plan, int T,
+static cudaError_t launch_one(const StepParams<typename Codec<S>::Real>& p, const TileLaunch& l, const TilePlan& plan, int steps,
                               cudaStream_t s) {
     static_assert(Sh::smem_bytes() <= 227 * 1024, "a tile's regions must fit into shared memory");
     // what the kernel's indices rely on
+    const int T = std::min(steps, plan.steps), total = steps;
     const bool fits = T >= 2 && T % 2 == 0 && T <= Sh::kMaxSteps && plan.h >= 2 && plan.h % 2 == 0 &&
                       plan.h + 2 * Sh::D * T <= Sh::MAXR && p.nx >= Sh::PX && p.ny >= plan.h + 2 * Sh::D * T &&
                       ((size_t)p.nx * sizeof(S)) % G == 0 && 9ULL * (unsigned long long)p.N <= (1ULL << 32);
-    if (!fits) return cudaErrorInvalidValue;
+    if (!fits || total % 2) return cudaErrorInvalidValue;
     auto kern = k_step_tiles<S, ABS, Sh, G>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::smem_bytes());
     if (e != cudaSuccess) return e;
     const int tx = (p.nx + Sh::W - 1) / Sh::W, ty = (p.ny + plan.h - 1) / plan.h;
+    const bool rounds = total > T;
+    // without moving warps a CTA has one tile; in rounds, every CTA waits for others
+    if (Sh::MOVERS ? rounds : tx * ty > l.sms) return cudaErrorInvalidValue;
+    if (rounds) {
+        const int depth = Sh::D * T, side = std::max(0, plan.h - 2 * depth);
+        const int ring = std::min(plan.h, 2 * depth) * Sh::W + side * std::min(Sh::W, 2 * Sh::HALO);
+        const size_t bytes = 2 * sizeof(uint4) * (size_t)(tx * ty) * Sh::kRecords * (size_t)l.ex.cap;
+        if (!l.ex.records || !l.ex.rounds || ring > l.ex.cap || bytes > l.ex.bytes || ring > Sh::kMostRing ||
+            2 * depth * Sh::PX + plan.h * 2 * Sh::HALO > Sh::kMostHalo)
+            return cudaErrorInvalidValue;
+    }
     ClassMarks marks{};
     for (int k = 0; k < kMaxClasses; ++k) {
         const uint32_t fl = p.cls.flags[k];
@@ -48,22 +60,28 @@ static cudaError_t launch_one(const StepParams<typename Codec<S>::Real>& p, cons
         marks.zouhe |= (fl & (kZouHeVelXm | kZouHeRhoXp) ? 1u : 0u) << k;
     }
     if (Sh::SC && marks.outlet) return cudaErrorInvalidValue;  // no zero-gradient cells in Shan-Chen tiles
-    // a launch may be scheduled while the one before it drains (the kernel waits for its end itself)
+    // a launch may be scheduled while the one before it drains (the kernel waits for its end itself); one in rounds
+    // starts with all its CTAs or not at all
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    if (rounds) {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+    }
     cfg.gridDim = dim3((unsigned)std::min(tx * ty, l.sms));
     cfg.blockDim = dim3(Sh::BLOCK);
     cfg.dynamicSmemBytes = Sh::smem_bytes();
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p, plan.h, T, tx, tx * ty, marks, -0.0f, l.err);
+    return cudaLaunchKernelEx(&cfg, kern, p, plan.h, T, total, tx, tx * ty, marks, -0.0f, l.ex, l.err);
 }
 
 template <class S, bool ABS>
-static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, const TileLaunch& l, const TilePlan& plan, int T,
+static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, const TileLaunch& l, const TilePlan& plan, int steps,
                                cudaStream_t s) {
     constexpr int kWord = (int)sizeof(S);
     const size_t row = (size_t)p.nx * kWord;
@@ -71,18 +89,18 @@ static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, con
     auto by_piece = [&](auto sh) {
         using Sh = decltype(sh);
         if constexpr (kWord == 2 || !ABS) {
-            if (row % 16 == 0) return launch_one<S, ABS, Sh, 16>(p, l, plan, T, s);
+            if (row % 16 == 0) return launch_one<S, ABS, Sh, 16>(p, l, plan, steps, s);
         }
         if constexpr (kWord == 2) {
-            if (row % 4 == 0) return launch_one<S, ABS, Sh, 4>(p, l, plan, T, s);
+            if (row % 4 == 0) return launch_one<S, ABS, Sh, 4>(p, l, plan, steps, s);
         }
-        return launch_one<S, ABS, Sh, kWord>(p, l, plan, T, s);
+        return launch_one<S, ABS, Sh, kWord>(p, l, plan, steps, s);
     };
     if constexpr (kWord <= 4 && !ABS) {
         if (plan.kind == kTilesShanChen) return by_piece(ShanChenShape<S>{});
     }
     if constexpr (kWord >= 4 && !ABS) {
-        if (plan.kind == kTilesStream && row % 16 == 0) return launch_one<S, ABS, StreamShape<S, true>, 16>(p, l, plan, T, s);
+        if (plan.kind == kTilesStream && row % 16 == 0) return launch_one<S, ABS, StreamShape<S, true>, 16>(p, l, plan, steps, s);
     }
     if constexpr (kWord == 4 && !ABS) {
         if (plan.kind == kTilesPieces) return by_piece(StreamShape<S, false>{});
@@ -92,24 +110,38 @@ static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, con
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int T, cudaStream_t s) {
+int tile_launch_steps(const TilePlan& plan) {
+    return plan.kind == kTilesSmall || plan.kind == kTilesMid ? 4096 : plan.steps;
+}
+
+TileExchange tile_exchange(const lbm_desc& d, const TilePlan& plan) {
+    TileExchange e;
+    if (plan.kind != kTilesSmall && plan.kind != kTilesMid) return e;
+    const int word = storage_bytes(d.storage), w = plan.kind == kTilesSmall ? 16 : 64;
+    const int halo = plan.kind == kTilesSmall ? 8 : (word == 2 ? 8 : 4), depth = plan.steps;
+    const int tiles = ((d.nx + w - 1) / w) * ((d.ny + plan.h - 1) / plan.h);
+    e.cap = std::min(plan.h, 2 * depth) * w + std::max(0, plan.h - 2 * depth) * std::min(w, 2 * halo);
+    e.bytes = 2 * sizeof(uint4) * (size_t)tiles * (size_t)((9 * word + 11) / 12) * (size_t)e.cap;
+    return e;
+}
+
+cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int steps, cudaStream_t s) {
     const bool abs_arith = d.arithmetic == LBM_ARITH_ABSOLUTE;
     switch (d.storage) {
         case LBM_F32:
-            return abs_arith ? launch_kind<float, true>(l.pf, l, plan, T, s) : launch_kind<float, false>(l.pf, l, plan, T, s);
-        case LBM_F16S: return launch_kind<__half, false>(l.pf, l, plan, T, s);
-        case LBM_BF16S: return launch_kind<__nv_bfloat16, false>(l.pf, l, plan, T, s);
+            return abs_arith ? launch_kind<float, true>(l.pf, l, plan, steps, s) : launch_kind<float, false>(l.pf, l, plan, steps, s);
+        case LBM_F16S: return launch_kind<__half, false>(l.pf, l, plan, steps, s);
+        case LBM_BF16S: return launch_kind<__nv_bfloat16, false>(l.pf, l, plan, steps, s);
         default:
-            return abs_arith ? launch_kind<double, true>(l.pd, l, plan, T, s) : launch_kind<double, false>(l.pd, l, plan, T, s);
+            return abs_arith ? launch_kind<double, true>(l.pd, l, plan, steps, s) : launch_kind<double, false>(l.pd, l, plan, steps, s);
     }
 }
 
 // When tiles are faster than single steps (measured on B200, lid cavities, us per step, single -> tiles).
-// - BGK lattices that one wave of CTAs covers: a launch of T steps then costs about 2 us of launch and drain, 2 us of
-//   moves and T short steps.  Small tiles first, for more CTAs: 96^2 FP32 1.4 -> 0.9, 128^2 1.8 -> 1.0, 192^2
-//   (16-row tiles, 4 steps) 3.5 -> 1.5; then 64-column tiles: 256^2 4.7 -> 1.6, 512^2 4.6 -> 3.3, 1000 x 300 5.0 ->
-//   3.7 (FP16S 512^2 6.2 -> 4.0, 1000 x 300 5.0 -> 4.0).  FP64 collisions take twice as long, so only up to
-//   14 rows: 256^2 4.1 -> 2.7, 384^2 (16 rows) 4.3 -> 4.2, 512^2 5.3 -> 6.3.
+// - BGK lattices that one wave of CTAs covers, in rounds of T steps: about 1.2 us a round for the exchange and T short
+//   steps.  Small tiles first, for more CTAs: 96^2 FP32 1.4 -> 0.7, 128^2 1.8 -> 0.8, 192^2 (16-row tiles, 4 steps)
+//   2.5 -> 1.1; then 64-column tiles: 256^2 2.9 -> 1.3, 512^2 4.6 -> 2.6, 1000 x 300 4.3 -> 2.8; FP16S 192^2 2.7 -> 1.2,
+//   512^2 5.2 -> 3.3, 1000 x 300 5.0 -> 3.5; FP64 256^2 3.3 -> 2.2, 384^2 4.0 -> 3.35, 640 x 400 (32 rows) 5.35 -> 4.75.
 // - FP32 BGK in L2, several waves: a wave of h-row tiles takes 2.3 (h + 6) / 36 us, a launch 1.4, a single step 1.5
 //   and its cells at 107 G/s, which decides (1024 x 512 6.6 -> 6.2, 1024^2 11.2 -> 10.6; 1500 x 451 8.0 -> 8.7 stays
 //   single).  16-bit words gain nothing there (1024 x 512 FP16S 7.4 -> 7.2, 1024^2 11.4 -> 13.3).
@@ -152,7 +184,7 @@ TilePlan plan_tiles(const lbm_desc& d, int sms) {
     }
     if (const int h = one_wave(16, 8)) return plan(kTilesSmall, 32, h, 8, 8);
     if (const int h = one_wave(16, 16)) return plan(kTilesSmall, 32, h, 4, 4);
-    if (const int h = one_wave(64, word == 8 ? 14 : 36)) return plan(kTilesMid, mid_px, h, 4, 4);
+    if (const int h = one_wave(64, word == 8 ? 32 : 36)) return plan(kTilesMid, mid_px, h, 4, 4);
     if (abs_arith) return TilePlan{};
     const long long bytes = 2LL * 9 * word * d.nx * d.ny;  // both buffers
     if (word == 4 && whole && bytes > 80000000LL) return plan(kTilesStream, mid_px, 34, 4, 4);

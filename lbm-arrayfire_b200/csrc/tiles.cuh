@@ -27,9 +27,18 @@
 // many tiles, four warps of their own move whole rows by bulk copies beside the computing ones (one warp
 // issues a bulk copy every 58 cycles, four keep up).
 //
-// Measured on B200 (us per step, one-step kernels -> tiles, lid cavities): 128^2 FP32 1.74 -> 0.85 and FP16S
-// 2.07 -> 1.06 (8 steps of 16 x 8 tiles); 1024 x 256 channel FP32 4.5 -> 3.5, FP16S 5.2 -> 4.2; 4096^2 FP32 188 ->
-// 118 (142 GLUPS; at one crossing per step HBM allows 91).
+// Rounds.  Where one wave of CTAs covers the lattice, tiles stay in their CTAs for a whole run (a cooperative launch:
+// all CTAs are resident).  After T steps a CTA gives the cells within T of its tile's edges to its neighbours and
+// takes its own halo from them, instead of ending the launch (2 us of drain and launch) and moving the
+// whole tile (2 us).  The words travel in 16-byte records that carry the number of their round, so the reader
+// polls the data itself: one way through L2, 1.0 to 1.3 us a round, without a fence and a flag (flags: 2.2 to 3.2 us).
+// Two slots of records by turns are enough: a CTA writes a slot again only after it has its neighbours' next records,
+// which they sent after reading the last ones.  Waits are bounded (two seconds, then an error).
+//
+// Measured on B200 (us per step, one-step kernels -> one launch per T steps -> rounds, lid cavities): 128^2 FP32 1.74 ->
+// 0.90 -> 0.77 and FP16S 2.07 -> 1.03 -> 0.91 (8 steps of 16 x 8 tiles); 512^2 FP32 4.6 -> 3.3 -> 2.65; 1024 x 256 channel
+// FP32 4.5 -> 3.6 -> 3.2; 1000 x 300 channel FP16S 5.2 -> 4.4 -> 4.1; many tiles a CTA: 4096^2 FP32 188 -> 118 (142
+// GLUPS; at one crossing per step HBM allows 91).
 //
 // The cell update is the other kernels' (bgk_collide, codecs and random words, with the step counter advanced
 // by T), so the results are bit-identical to single steps.  A launch leaves the state after T steps in
@@ -278,7 +287,13 @@ struct TileShape {
     static constexpr size_t kPsi = kPop + (size_t)NBUF * BUF * sizeof(S);
     static constexpr size_t kCls = kPsi + (SC ? (size_t)(MAXR * PX + 8) * sizeof(typename Codec<S>::Real) : 0);
     static constexpr size_t kClsBytes = (size_t)(MAXR * PX + 15) / 16 * 16;
-    static constexpr size_t smem_bytes() { return kCls + NBUF * kClsBytes; }
+    // rounds (no MOVERS): the cells that a tile gives to others, and its halo
+    static constexpr int kRecords = (9 * (int)sizeof(S) + 11) / 12;
+    static constexpr int kMostHalo = (PX * 2 * D * kMaxSteps + (MAXR - 2 * D * kMaxSteps) * 2 * HALO);
+    static constexpr int kMostRing = 2 * D * kMaxSteps * W + MAXR * 2 * HALO < W * MAXR ? 2 * D * kMaxSteps * W + MAXR * 2 * HALO : W * MAXR;
+    static constexpr size_t kEx = kCls + NBUF * kClsBytes;
+    static constexpr size_t kRingBytes = MOVERS ? 0 : ((size_t)kMostRing * 2 + 15) / 16 * 16;
+    static constexpr size_t smem_bytes() { return kEx + kRingBytes + (MOVERS ? 0 : (size_t)kMostHalo * 8); }
 };
 
 // bgk_collide out of line, for the rare cells that the packed collision leaves (Zou-He): keeps the loop short.
@@ -297,15 +312,29 @@ struct TilePlan {
     int h = 0;      // rows of a tile (even)
     int steps = 0;  // steps per launch (even)
 };
+// What tiles that stay in their CTAs exchange between rounds (zeroed when allocated; one lattice's own).
+// records: for each tile and cell of its border the nine words, three to a 16-byte record whose fourth word is
+// the number of the round that wrote it; two slots, by rounds.
+struct TileExchange {
+    uint4* records = nullptr;    // [2][tiles][records of a cell][cap]
+    unsigned* rounds = nullptr;  // [tiles] exchanges behind each tile
+    int cap = 0;                 // cells of a tile's border, at most
+    size_t bytes = 0;            // of the records
+};
 struct TileLaunch {
     StepParams<float> pf;
     StepParams<double> pd;
     int* err;
+    TileExchange ex;
     int sms;
 };
 // The plan of a D2Q9 BGK or Shan-Chen lattice on a device of `sms` SMs (kTilesNone: single steps are faster).
 TilePlan plan_tiles(const lbm_desc& d, int sms);
-cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int T, cudaStream_t s);
+// Most steps of one launch (where plan.steps is less: in rounds).
+int tile_launch_steps(const TilePlan& plan);
+// The exchange that launches in rounds of this plan need (cap and bytes; 0: none).
+TileExchange tile_exchange(const lbm_desc& d, const TilePlan& plan);
+cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan& plan, int steps, cudaStream_t s);
 
 // Two adjacent words.
 template <class S>
@@ -326,15 +355,45 @@ __device__ __forceinline__ void bulk_store(void* dst_gmem, const void* src_smem,
                  : "memory");
 }
 
-// One tile launch: tiles of W x h cells, T (even, D T <= HALO) steps.  nx >= PX and ny >= h + 2 D T
+// Place of cell (lx, ly) of a w x h tile in the order of its border (the cells within `depth` rows or `halo` columns
+// of its edges): the rows at both ends, then the rest of the columns; -1: an inner cell.
+__host__ __device__ inline int ring_index(int lx, int ly, int w, int h, int halo, int depth) {
+    const int rows = h < 2 * depth ? h : 2 * depth, cols = w < 2 * halo ? w : 2 * halo;
+    const int top = h < depth ? h : depth, left = w < halo ? w : halo;
+    if (ly < top) return ly * w + lx;
+    if (ly >= h - (rows - top)) return (ly - (h - rows)) * w + lx;
+    if (lx >= left && lx < w - (cols - left)) return -1;
+    return rows * w + (ly - top) * cols + (lx < left ? lx : lx - (w - cols));
+}
+
+// Records are read and written whole (128-bit accesses are single-copy atomic): one with the right number is there.
+__device__ __forceinline__ void store_record(uint4* to, const uint4& r) {
+    asm volatile(
+        "{\n\t.reg .b128 r;\n\t.reg .b64 lo, hi;\n\tmov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\tmov.b128 r, {lo, hi};\n\t"
+        "st.relaxed.gpu.global.b128 [%0], r;\n\t}" ::"l"(to),
+        "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
+        : "memory");
+}
+__device__ __forceinline__ uint4 load_record(const uint4* from) {
+    uint4 r;
+    asm volatile(
+        "{\n\t.reg .b128 r;\n\t.reg .b64 lo, hi;\n\tld.relaxed.gpu.global.b128 r, [%4];\n\tmov.b128 {lo, hi}, r;\n\t"
+        "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+        : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+        : "l"(from)
+        : "memory");
+    return r;
+}
+
+// One tile launch: tiles of W x h cells, `total` steps: T (even, D T <= HALO), or (no MOVERS, a tile a CTA) rounds of T.  nx >= PX and ny >= h + 2 D T
 // (host-checked): every region cell wraps at most once.  CTAs walk the tiles with a stride.  A thread takes
 // two cells at a time (PX and h are even).
 // G: bytes of the pieces that regions and tiles move in, 16, 8, 4 or (16-bit words) 2: every row of the
 // lattice starts on a multiple of it.
 template <class S, bool ABS, class Sh, int G>
 __global__ void __launch_bounds__(Sh::BLOCK, 1)
-    k_step_tiles(const __grid_constant__ StepParams<typename Codec<S>::Real> p, int h, int T, int tiles_x, int tiles,
-                 const ClassMarks marks, float minus_zero, int* __restrict__ err) {
+    k_step_tiles(const __grid_constant__ StepParams<typename Codec<S>::Real> p, int h, int T, int total, int tiles_x, int tiles,
+                 const ClassMarks marks, float minus_zero, const TileExchange ex, int* __restrict__ err) {
     using L = D2Q9;
     using R = typename Codec<S>::Real;
     constexpr int Q = 9, PX = Sh::PX, PLANE = Sh::PLANE, THREADS = Sh::THREADS, HALO = Sh::HALO, W = Sh::W, NBUF = Sh::NBUF;
@@ -540,7 +599,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
     if constexpr (k16) {
         if (p.sr) {
             t0 = p.tick[p.parity];
-            if ((blockIdx.x | (unsigned)tid) == 0) p.tick[p.parity ^ 1] = t0 + (unsigned)T;
+            if ((blockIdx.x | (unsigned)tid) == 0) p.tick[p.parity ^ 1] = t0 + (unsigned)total;
         }
     }
     uint32_t next_cls[kClsWords], seen = 0;
@@ -574,15 +633,57 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
         } else if (!kMove) {
             barrier();
         }
+        unsigned base = 0;
+        int ring = 0, halo = 0;
+        uint16_t* const ring_k = reinterpret_cast<uint16_t*>(smem + Sh::kEx);
+        uint2* const halo_k = reinterpret_cast<uint2*>(smem + Sh::kEx + Sh::kRingBytes);
+        if (!kMove && total > T) {
+            // Rounds.  ring_k: the region's index of each cell that others need, in the order of its records;
+            // halo_k: for each cell of the halo its first record and its index.
+            base = ex.rounds[n];
+            auto width = [&](int t) { return nx - t * W < W ? nx - t * W : W; };
+            auto height = [&](int t) { return ny - t * h < h ? ny - t * h : h; };
+            const int w = width(tx), hh = height(ty);
+            auto ends = [&](int size, int most) { return size < 2 * most ? size : 2 * most; };
+            ring = ends(hh, depth) * w + (hh - ends(hh, depth)) * ends(w, HALO);
+            for (int q = tid; q < hh * w; q += THREADS) {
+                const int ly = q / w, lx = q - ly * w;
+                const int at = ring_index(lx, ly, w, hh, HALO, depth);
+                if (at >= 0) ring_k[at] = (uint16_t)((ly + depth) * PX + lx + HALO);
+            }
+            const int full = w + 2 * HALO, caps = 2 * depth * full;
+            halo = caps + hh * 2 * HALO;
+            for (int m = tid; m < halo; m += THREADS) {
+                int ly, lx;
+                if (m < caps) {
+                    ly = m / full;
+                    lx = m - ly * full;
+                    if (ly >= depth) ly += hh;
+                } else {
+                    ly = (m - caps) / (2 * HALO);
+                    lx = m - caps - ly * 2 * HALO;
+                    ly += depth;
+                    if (lx >= HALO) lx += w;
+                }
+                const uint32_t c = cell_of(x0, y0, ly * PX + lx);
+                const int y = (int)(c / (uint32_t)nx), x = (int)(c - (uint32_t)y * (uint32_t)nx);
+                const int sx = x / W, sy = y / h;
+                const int at = ring_index(x - sx * W, y - sy * h, width(sx), height(sy), HALO, depth);
+                halo_k[m] = uint2{(uint32_t)((sy * tiles_x + sx) * Sh::kRecords) * (uint32_t)ex.cap + (uint32_t)at,
+                                  (uint32_t)(ly * PX + lx)};
+            }
+            barrier();
+        }
         // the next tile's classes travel while this one is computed
         if (kMove && classes && n + stride < tiles) get_classes(n + stride, next_cls);
 
+        int before = 0;  // steps behind
         // One step.  AROUND (odd t): reads and writes the neighbours' words; else the cell's own.
         auto step = [&](auto Around, auto Special, int t) {
             constexpr bool around = decltype(Around)::value, SPECIAL = decltype(Special)::value;
             Rounding rnd{0u, false};
             if constexpr (k16) {
-                if (p.sr) rnd = Rounding{seed_of_step(t0 + (unsigned)(t - 1)), true};
+                if (p.sr) rnd = Rounding{seed_of_step(t0 + (unsigned)((kMove ? 0 : before) + t - 1)), true};
             }
             // the two cells of a thread: adjacent, or (FP32 and FP64 words around, where adjacent cells would
             // meet in a bank) half the rows apart
@@ -797,21 +898,89 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
         };
         auto steps = [&](auto Special) {
 #pragma unroll 1
-            for (int t = 1; t < T; t += 2) {
+            for (int t = 1; t < (kMove ? T : min(T, total - before)); t += 2) {
                 step(std::true_type{}, Special, t);
                 step(std::false_type{}, Special, t + 1);
             }
         };
-        if (kind)
-            steps(std::true_type{});
-        else
-            steps(std::false_type{});
+        int r = 0;  // rounds behind
+#pragma unroll 1
+        while (true) {
+            if (kind)
+                steps(std::true_type{});
+            else
+                steps(std::false_type{});
+            if constexpr (kMove) break;
+            before += T;
+            if (before >= total) break;
+            ++r;
+            const unsigned tag = base + (unsigned)r;
+            const uint32_t slot = (tag & 1u) * (uint32_t)(tiles * Sh::kRecords) * (uint32_t)ex.cap;
+            for (int q = tid; q < ring; q += THREADS) {
+                const S* const at = pop + ring_k[q];
+                uint32_t wd[3 * Sh::kRecords] = {};
+                static_for<Q>([&](auto I) {
+                    constexpr int i = I;
+                    const S v = at[i * PLANE];
+                    if constexpr (sizeof(S) == 2)
+                        wd[i / 2] |= (uint32_t)*reinterpret_cast<const uint16_t*>(&v) << (16 * (i & 1));
+                    else if constexpr (sizeof(S) == 4)
+                        wd[i] = __float_as_uint((float)v);
+                    else {
+                        wd[2 * i] = (uint32_t)__double2loint((double)v);
+                        wd[2 * i + 1] = (uint32_t)__double2hiint((double)v);
+                    }
+                });
+                uint4* const to = ex.records + slot + (uint32_t)(n * Sh::kRecords) * (uint32_t)ex.cap + q;
+                static_for<Sh::kRecords>([&](auto J) {
+                    constexpr int j = J;
+                    store_record(to + j * ex.cap, uint4{wd[3 * j], wd[3 * j + 1], wd[3 * j + 2], tag});
+                });
+            }
+            bool late = false;
+            for (int m = tid; m < halo; m += THREADS) {
+                const uint2 cell = halo_k[m];
+                const uint4* const from = ex.records + slot + cell.x;
+                uint4 rec[Sh::kRecords];
+                static_for<Sh::kRecords>([&](auto J) { rec[J] = load_record(from + J * ex.cap); });
+                const long long c0 = clock64();
+                while (true) {
+                    int missing = -1;
+                    static_for<Sh::kRecords>([&](auto J) { missing = rec[J].w != tag ? (int)J : missing; });
+                    if (missing < 0 || late) break;
+                    while (load_record(from + missing * ex.cap).w != tag)
+                        if (clock64() - c0 > (1LL << 32)) {
+                            late = true;
+                            break;
+                        }
+                    static_for<Sh::kRecords>([&](auto J) { rec[J] = load_record(from + J * ex.cap); });
+                }
+                S* const at = pop + cell.y;
+                uint32_t wd[3 * Sh::kRecords];
+                static_for<Sh::kRecords>([&](auto J) {
+                    wd[3 * J] = rec[J].x;
+                    wd[3 * J + 1] = rec[J].y;
+                    wd[3 * J + 2] = rec[J].z;
+                });
+                static_for<Q>([&](auto I) {
+                    constexpr int i = I;
+                    if constexpr (sizeof(S) == 2)
+                        reinterpret_cast<uint16_t*>(at)[i * PLANE] = (uint16_t)(wd[i / 2] >> (16 * (i & 1)));
+                    else if constexpr (sizeof(S) == 4)
+                        at[i * PLANE] = S(__uint_as_float(wd[i]));
+                    else
+                        at[i * PLANE] = S(__hiloint2double((int)wd[2 * i + 1], (int)wd[2 * i]));
+                });
+            }
+            if (late) atomicExch(err, kRowPipeTimeout);
+            if (any(late)) return;
+        }
+        if (!kMove && total > T && tid == 0) ex.rounds[n] = base + (unsigned)r;
         if constexpr (kMove) {
             if (tid == 0) mbar_arrive(&done[b]);
             if (classes && n + stride < tiles) seen = put_classes(next_cls, b ^ 1);
         } else {
-            pieces_out(n, 0, tid, THREADS);
-            if (n + stride < tiles) barrier();
+            pieces_out(n, 0, tid, THREADS);  // (one tile a CTA)
         }
     }
 }
