@@ -37,7 +37,7 @@
 //
 // Measured on B200 (us per step, one-step kernels -> one launch per T steps -> rounds, lid cavities): 128^2 FP32 1.74 ->
 // 0.90 -> 0.77 and FP16S 2.07 -> 1.03 -> 0.91 (8 steps of 16 x 8 tiles); 512^2 FP32 4.6 -> 3.3 -> 2.65; 1024 x 256 channel
-// FP32 4.5 -> 3.6 -> 3.2; 1000 x 300 channel FP16S 5.2 -> 4.4 -> 4.1; many tiles a CTA: 4096^2 FP32 188 -> 118 (142
+// FP32 4.5 -> 3.6 -> 3.0; 1000 x 300 channel FP16S 5.2 -> 4.4 -> 3.8; many tiles a CTA: 4096^2 FP32 188 -> 118 (142
 // GLUPS; at one crossing per step HBM allows 91).
 //
 // The cell update is the other kernels' (bgk_collide, codecs and random words, with the step counter advanced
@@ -291,7 +291,8 @@ struct TileShape {
     static constexpr int kRecords = (9 * (int)sizeof(S) + 11) / 12;
     static constexpr int kMostHalo = (PX * 2 * D * kMaxSteps + (MAXR - 2 * D * kMaxSteps) * 2 * HALO);
     static constexpr int kMostRing = 2 * D * kMaxSteps * W + MAXR * 2 * HALO < W * MAXR ? 2 * D * kMaxSteps * W + MAXR * 2 * HALO : W * MAXR;
-    static constexpr size_t kEx = kCls + NBUF * kClsBytes;
+    static constexpr size_t kOutlets = kCls + NBUF * kClsBytes;  // words of class bytes with zero-gradient cells
+    static constexpr size_t kEx = kOutlets + (SC ? 0 : ((size_t)(MAXR * PX / 4) * 2 + 15) / 16 * 16);
     static constexpr size_t kRingBytes = MOVERS ? 0 : ((size_t)kMostRing * 2 + 15) / 16 * 16;
     static constexpr size_t smem_bytes() { return kEx + kRingBytes + (MOVERS ? 0 : (size_t)kMostHalo * 8); }
 };
@@ -633,6 +634,28 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
         } else if (!kMove) {
             barrier();
         }
+        // the words of class bytes with zero-gradient cells, last first
+        uint16_t* const outlet = reinterpret_cast<uint16_t*>(smem + Sh::kOutlets);
+        int outlets = 0;
+        if (!SC && (kind & kMarkOutlet)) {
+            int* const found = reinterpret_cast<int*>(smem + 32);
+            if (tid < 32) {
+                const int words_ = rows * (PX / 4);
+                int sum = 0;
+#pragma unroll 4
+                for (int from = 0; from < words_; from += 32) {
+                    const int m = words_ - 1 - from - tid;
+                    const uint32_t c = m >= 0 ? reinterpret_cast<const uint32_t*>(cls_s)[m] : 0u;
+                    const bool has = (c & (kMarkOutlet * 0x01010101u)) != 0;
+                    const unsigned all = __ballot_sync(0xffffffffu, has);
+                    if (has) outlet[sum + __popc(all & ((1u << tid) - 1u))] = (uint16_t)m;
+                    sum += __popc(all);
+                }
+                if (tid == 0) *found = sum;
+            }
+            barrier();
+            outlets = *found;
+        }
         unsigned base = 0;
         int ring = 0, halo = 0;
         uint16_t* const ring_k = reinterpret_cast<uint16_t*>(smem + Sh::kEx);
@@ -697,36 +720,32 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                 // A zero-gradient cell's c_x = -1 populations are f_i(x, y - c_iy) of its own column, which
                 // the cell to its left reads and overwrites.  They are copied to where the cell itself
                 // reads, which no other cell touches in this step.
-                if (kind & kMarkOutlet) {
-                    const int w0 = first / 4, w1 = (rows * PX - first) / 4;
-                    for (int base = w0; base < w1; base += THREADS) {
-                        const int m = base + tid;
-                        const uint32_t word = m < w1 ? reinterpret_cast<const uint32_t*>(cls_s)[m] : 0u;
-                        const bool mine = (word & (kMarkOutlet * 0x01010101u)) != 0;
-                        S zg[4][3];
-                        if (mine) {
-                            static_for<4>([&](auto U) {
-                                static_for<3>([&](auto J) {
-                                    constexpr int u = U, i = J == 0 ? 3 : (J == 1 ? 6 : 7);
-                                    const int k = 4 * m + u;
-                                    zg[u][J] = around ? pop[i * PLANE + k - L::cy(i) * PX] : pop[L::opp(i) * PLANE + k - 1];
-                                });
+                // Cell k's copies go where those of cell k + 1 come from, so the last cells are first.
+                for (int from = 0; from < outlets; from += THREADS) {
+                    const int m = from + tid < outlets ? (int)outlet[from + tid] : -1;
+                    const bool mine = m >= first / 4 && m < (rows * PX - first) / 4;
+                    const uint32_t word = mine ? reinterpret_cast<const uint32_t*>(cls_s)[m] : 0u;
+                    S zg[4][3];
+                    static_for<4>([&](auto U) {
+                        constexpr int u = U;
+                        if ((word >> (8 * u)) & kMarkOutlet)
+                            static_for<3>([&](auto J) {
+                                constexpr int i = J == 0 ? 3 : (J == 1 ? 6 : 7);
+                                const int k = 4 * m + u;
+                                zg[u][J] = around ? pop[i * PLANE + k - L::cy(i) * PX] : pop[L::opp(i) * PLANE + k - 1];
                             });
-                        }
-                        barrier();
-                        if (mine) {
-                            static_for<4>([&](auto U) {
-                                constexpr int u = U;
-                                if ((word >> (8 * u)) & kMarkOutlet)
-                                    static_for<3>([&](auto J) {
-                                        constexpr int i = J == 0 ? 3 : (J == 1 ? 6 : 7);
-                                        const int k = 4 * m + u;
-                                        (around ? pop[i * PLANE + k - L::cy(i) * PX + 1] : pop[L::opp(i) * PLANE + k]) = zg[u][J];
-                                    });
+                    });
+                    barrier();
+                    static_for<4>([&](auto U) {
+                        constexpr int u = U;
+                        if ((word >> (8 * u)) & kMarkOutlet)
+                            static_for<3>([&](auto J) {
+                                constexpr int i = J == 0 ? 3 : (J == 1 ? 6 : 7);
+                                const int k = 4 * m + u;
+                                (around ? pop[i * PLANE + k - L::cy(i) * PX + 1] : pop[L::opp(i) * PLANE + k]) = zg[u][J];
                             });
-                        }
-                        barrier();
-                    }
+                    });
+                    barrier();
                 }
             }
             auto value = [&](S w, auto I) -> R {

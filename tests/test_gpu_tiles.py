@@ -66,6 +66,9 @@ def same(kind, nx, ny, storage, arithmetic, runs):
     (0, 260, 190),          # mid shape, the reference's channel
     (1, 301, 199),          # mid shape, rows that start anywhere
     ("outlets", 96, 80),
+    ("outlets", 300, 200),  # more zero-gradient cells than threads
+    ("lid", 129, 105),      # last tiles of one column and one row
+    (1, 257, 199),
 ])
 def test_tiles_equal_plain_steps(kind, nx, ny, storage):
     same(kind, nx, ny, storage, DEV, (1, 2, 3, 4, 9, 10, 31))
@@ -83,6 +86,7 @@ def test_tiles_equal_plain_steps_in_absolute_arithmetic(kind, nx, ny, storage):
     (lb.F32, "periodic", 1068, 1067),  # a short last tile in x and y
     (lb.F32, 1, 1501, 1201),           # rows that start anywhere: moved in pieces
     (lb.F64, 1, 1030, 1000),           # streamed by bulk copies
+    (lb.F32, "outlets", 1200, 1000),
 ])
 def test_many_tiles_per_cta(storage, kind, nx, ny):
     same(kind, nx, ny, storage, DEV, (7, 12))
