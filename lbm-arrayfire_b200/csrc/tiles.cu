@@ -46,10 +46,10 @@ static cudaError_t launch_one(const StepParams<typename Codec<S>::Real>& p, cons
     if (Sh::MOVERS ? rounds : tx * ty > l.sms) return cudaErrorInvalidValue;
     if (rounds) {
         const int depth = Sh::D * T, side = std::max(0, plan.h - 2 * depth);
-        const int ring = std::min(plan.h, 2 * depth) * Sh::W + side * std::min(Sh::W, 2 * Sh::HALO);
+        const int ring = std::min(plan.h, 2 * depth) * Sh::W + side * std::min(Sh::W, 2 * depth);
         const size_t bytes = 2 * sizeof(uint4) * (size_t)(tx * ty) * Sh::kRecords * (size_t)l.ex.cap;
         if (!l.ex.records || !l.ex.rounds || ring > l.ex.cap || bytes > l.ex.bytes || ring > Sh::kMostRing ||
-            2 * depth * Sh::PX + plan.h * 2 * Sh::HALO > Sh::kMostHalo)
+            2 * depth * (Sh::W + 2 * depth) + plan.h * 2 * depth > Sh::kMostHalo)
             return cudaErrorInvalidValue;
     }
     ClassMarks marks{};
@@ -118,9 +118,9 @@ TileExchange tile_exchange(const lbm_desc& d, const TilePlan& plan) {
     TileExchange e;
     if (plan.kind != kTilesSmall && plan.kind != kTilesMid) return e;
     const int word = storage_bytes(d.storage), w = plan.kind == kTilesSmall ? 16 : 64;
-    const int halo = plan.kind == kTilesSmall ? 8 : (word == 2 ? 8 : 4), depth = plan.steps;
+    const int depth = plan.steps;
     const int tiles = ((d.nx + w - 1) / w) * ((d.ny + plan.h - 1) / plan.h);
-    e.cap = std::min(plan.h, 2 * depth) * w + std::max(0, plan.h - 2 * depth) * std::min(w, 2 * halo);
+    e.cap = std::min(plan.h, 2 * depth) * w + std::max(0, plan.h - 2 * depth) * std::min(w, 2 * depth);
     e.bytes = 2 * sizeof(uint4) * (size_t)tiles * (size_t)((9 * word + 11) / 12) * (size_t)e.cap;
     return e;
 }
@@ -138,7 +138,7 @@ cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan&
 }
 
 // When tiles are faster than single steps (measured on B200, lid cavities, us per step, single -> tiles).
-// - BGK lattices that one wave of CTAs covers, in rounds of T steps: about 1.2 us a round for the exchange and T short
+// - BGK lattices that one wave of CTAs covers, in rounds of T steps: about 2 us a round for the exchange and T short
 //   steps.  Small tiles first, for more CTAs: 96^2 FP32 1.4 -> 0.7, 128^2 1.8 -> 0.8, 192^2 (16-row tiles, 4 steps)
 //   2.5 -> 1.1; then 64-column tiles: 256^2 2.9 -> 1.3, 512^2 4.6 -> 2.6, 1000 x 300 4.3 -> 2.8; FP16S 192^2 2.7 -> 1.2,
 //   512^2 5.2 -> 3.3, 1000 x 300 5.0 -> 3.5; FP64 256^2 3.3 -> 2.2, 384^2 4.0 -> 3.35, 640 x 400 (32 rows) 5.35 -> 4.75.

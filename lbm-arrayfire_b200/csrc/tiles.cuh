@@ -31,7 +31,9 @@
 // all CTAs are resident).  After T steps a CTA gives the cells within T of its tile's edges to its neighbours and
 // takes its own halo from them, instead of ending the launch (2 us of drain and launch) and moving the
 // whole tile (2 us).  The words travel in 16-byte records that carry the number of their round, so the reader
-// polls the data itself: one way through L2, 1.0 to 1.3 us a round, without a fence and a flag (flags: 2.2 to 3.2 us).
+// polls the data itself, without a fence and a flag: 1.6 us a round for 16-column tiles, 2.1 us for 64-column ones
+// (flags: 2.2 and 3.2 us; records sent from the last step's registers, in divergent stores, 2.7 us; all of a thread's
+// records requested at once, of which most are not there yet, 2.3 us).
 // Two slots of records by turns are enough: a CTA writes a slot again only after it has its neighbours' next records,
 // which they sent after reading the last ones.  Waits are bounded (two seconds, then an error).
 //
@@ -289,8 +291,10 @@ struct TileShape {
     static constexpr size_t kClsBytes = (size_t)(MAXR * PX + 15) / 16 * 16;
     // rounds (no MOVERS): the cells that a tile gives to others, and its halo
     static constexpr int kRecords = (9 * (int)sizeof(S) + 11) / 12;
-    static constexpr int kMostHalo = (PX * 2 * D * kMaxSteps + (MAXR - 2 * D * kMaxSteps) * 2 * HALO);
-    static constexpr int kMostRing = 2 * D * kMaxSteps * W + MAXR * 2 * HALO < W * MAXR ? 2 * D * kMaxSteps * W + MAXR * 2 * HALO : W * MAXR;
+    static constexpr int kReach = 2 * D * kMaxSteps;
+    static constexpr int kMostHalo = (W + kReach) * kReach + (MAXR - kReach) * kReach;
+    static constexpr int kMostRing = kReach * W + (MAXR - kReach) * kReach < W * MAXR ? kReach * W + (MAXR - kReach) * kReach : W * MAXR;
+    static constexpr int kHaloTurns = (kMostHalo + THREADS - 1) / THREADS;
     static constexpr size_t kOutlets = kCls + NBUF * kClsBytes;  // words of class bytes with zero-gradient cells
     static constexpr size_t kEx = kOutlets + (SC ? 0 : ((size_t)(MAXR * PX / 4) * 2 + 15) / 16 * 16);
     static constexpr size_t kRingBytes = MOVERS ? 0 : ((size_t)kMostRing * 2 + 15) / 16 * 16;
@@ -356,11 +360,11 @@ __device__ __forceinline__ void bulk_store(void* dst_gmem, const void* src_smem,
                  : "memory");
 }
 
-// Place of cell (lx, ly) of a w x h tile in the order of its border (the cells within `depth` rows or `halo` columns
-// of its edges): the rows at both ends, then the rest of the columns; -1: an inner cell.
-__host__ __device__ inline int ring_index(int lx, int ly, int w, int h, int halo, int depth) {
-    const int rows = h < 2 * depth ? h : 2 * depth, cols = w < 2 * halo ? w : 2 * halo;
-    const int top = h < depth ? h : depth, left = w < halo ? w : halo;
+// Place of cell (lx, ly) of a w x h tile in the order of its border (the cells within `depth` of its edges): the rows
+// at both ends, then the rest of the columns; -1: an inner cell.
+__host__ __device__ inline int ring_index(int lx, int ly, int w, int h, int depth) {
+    const int rows = h < 2 * depth ? h : 2 * depth, cols = w < 2 * depth ? w : 2 * depth;
+    const int top = h < depth ? h : depth, left = w < depth ? w : depth;
     if (ly < top) return ly * w + lx;
     if (ly >= h - (rows - top)) return (ly - (h - rows)) * w + lx;
     if (lx >= left && lx < w - (cols - left)) return -1;
@@ -667,15 +671,15 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
             auto width = [&](int t) { return nx - t * W < W ? nx - t * W : W; };
             auto height = [&](int t) { return ny - t * h < h ? ny - t * h : h; };
             const int w = width(tx), hh = height(ty);
-            auto ends = [&](int size, int most) { return size < 2 * most ? size : 2 * most; };
-            ring = ends(hh, depth) * w + (hh - ends(hh, depth)) * ends(w, HALO);
+            auto ends = [&](int size) { return size < 2 * depth ? size : 2 * depth; };
+            ring = ends(hh) * w + (hh - ends(hh)) * ends(w);
             for (int q = tid; q < hh * w; q += THREADS) {
                 const int ly = q / w, lx = q - ly * w;
-                const int at = ring_index(lx, ly, w, hh, HALO, depth);
+                const int at = ring_index(lx, ly, w, hh, depth);
                 if (at >= 0) ring_k[at] = (uint16_t)((ly + depth) * PX + lx + HALO);
             }
-            const int full = w + 2 * HALO, caps = 2 * depth * full;
-            halo = caps + hh * 2 * HALO;
+            const int full = w + 2 * depth, caps = 2 * depth * full;
+            halo = caps + hh * 2 * depth;
             for (int m = tid; m < halo; m += THREADS) {
                 int ly, lx;
                 if (m < caps) {
@@ -683,15 +687,16 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                     lx = m - ly * full;
                     if (ly >= depth) ly += hh;
                 } else {
-                    ly = (m - caps) / (2 * HALO);
-                    lx = m - caps - ly * 2 * HALO;
+                    ly = (m - caps) / (2 * depth);
+                    lx = m - caps - ly * 2 * depth;
                     ly += depth;
-                    if (lx >= HALO) lx += w;
+                    if (lx >= depth) lx += w;
                 }
+                lx += HALO - depth;
                 const uint32_t c = cell_of(x0, y0, ly * PX + lx);
                 const int y = (int)(c / (uint32_t)nx), x = (int)(c - (uint32_t)y * (uint32_t)nx);
                 const int sx = x / W, sy = y / h;
-                const int at = ring_index(x - sx * W, y - sy * h, width(sx), height(sy), HALO, depth);
+                const int at = ring_index(x - sx * W, y - sy * h, width(sx), height(sy), depth);
                 halo_k[m] = uint2{(uint32_t)((sy * tiles_x + sx) * Sh::kRecords) * (uint32_t)ex.cap + (uint32_t)at,
                                   (uint32_t)(ly * PX + lx)};
             }
@@ -957,21 +962,19 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                 });
             }
             bool late = false;
-            for (int m = tid; m < halo; m += THREADS) {
+            static_for<Sh::kHaloTurns>([&](auto U) {
+                const int m = tid + (int)U * THREADS;
+                if (m >= halo) return;
                 const uint2 cell = halo_k[m];
                 const uint4* const from = ex.records + slot + cell.x;
                 uint4 rec[Sh::kRecords];
                 static_for<Sh::kRecords>([&](auto J) { rec[J] = load_record(from + J * ex.cap); });
-                const long long c0 = clock64();
                 while (true) {
                     int missing = -1;
                     static_for<Sh::kRecords>([&](auto J) { missing = rec[J].w != tag ? (int)J : missing; });
                     if (missing < 0 || late) break;
-                    while (load_record(from + missing * ex.cap).w != tag)
-                        if (clock64() - c0 > (1LL << 32)) {
-                            late = true;
-                            break;
-                        }
+                    const long long c0 = clock64();
+                    while (!late && load_record(from + missing * ex.cap).w != tag) late = clock64() - c0 > (1LL << 32);
                     static_for<Sh::kRecords>([&](auto J) { rec[J] = load_record(from + J * ex.cap); });
                 }
                 S* const at = pop + cell.y;
@@ -990,7 +993,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                     else
                         at[i * PLANE] = S(__hiloint2double((int)wd[2 * i + 1], (int)wd[2 * i]));
                 });
-            }
+            });
             if (late) atomicExch(err, kRowPipeTimeout);
             if (any(late)) return;
         }
