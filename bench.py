@@ -822,18 +822,16 @@ def config_lines(torch, lb, args, dev, world):
             a.workload, a.steps, a.warmup = wl, steps, max(args.warmup, 3)
             a.kernel, a.block, a.dims, a.size = "auto", 0, "", 0
             d, lat, el, _ = measure(torch, lb, a, STORAGES[stn], dev, world)
-            fam = KERNEL_NAMES.get(lat.kernel(), "unknown")
+            launches, kernels = counted_launches(torch, lat, steps)
             lat.close()
             del lat
             rec[stn] = {"value": d.cells * steps / el / 1e6, "unit": "MLUPS", "ms_per_step": el * 1e3 / steps,
-                        "kernel_family": fam,
+                        "kernels": kernels, "launches_per_step": launches / steps,
                         "achieved_gbs": algorithmic_bytes_per_cell(d) * d.cells * steps / el / 1e9}
             rec["lattice"] = list(d.shape)
             mb = d.cells * d.q * storage_bytes(STORAGES[stn]) * 2 / 1e6
-            rec["l2"] = (f"L2-resident ({mb:.1f} MB of populations in both buffers at {stn}); no flush"
-                         if fam != "cluster" else
-                         f"resident in one thread-block cluster's shared memory ({mb:.1f} MB at {stn}) for up "
-                         f"to 4096 steps per launch; HBM/L2 only at launch start and end")
+            rec["l2"] = (f"L2-resident ({mb:.1f} MB of populations in both buffers at {stn}); no flush; several steps per "
+                         f"launch in shared memory where launches_per_step is below 1")
         rec[f"speedup_{st16}_vs_f32"] = rec[st16]["value"] / rec["f32"]["value"]
         rec["steps"] = steps
         out[wl] = rec
@@ -848,6 +846,18 @@ def config_lines(torch, lb, args, dev, world):
     return out
 
 
+def counted_launches(torch, lat, steps):
+    """Kernel launches of `steps` more steps of a lattice, and the kernels' names (outside any timed region)."""
+    import re
+
+    lat.sync()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        lat.step(steps)
+        lat.sync()
+    names = [e.name for e in prof.events() if "k_step" in e.name or "k_sc_psi" in e.name]
+    return len(names), sorted({re.search(r"k_\w+", n).group(0) for n in names})
+
+
 def run_ours(args, rank, world, local_rank):
     import torch
 
@@ -860,11 +870,12 @@ def run_ours(args, rank, world, local_rank):
 
     d, lat, el, clocks = measure(torch, lb, args, head_storage, dev, world, sample_clocks=(rank == 0))
     N = d.cells
-    # Shan-Chen: two launches per step, one with the one-pass kernel (the single-pass family); the
-    # cluster-resident family: one launch per 4096 steps
-    launches_per_step = 2 if d.collision == 2 and lat.kernel() != lb.KERNEL_ROWS else 1
-    if lat.kernel() == lb.KERNEL_CLUSTER:
-        launches_per_step = -(-args.steps // 4096) / args.steps
+    # one launch per step, except in two dimensions (several steps per launch on tiles, one per 4096 in a cluster,
+    # Shan-Chen's two passes), where the launches of as many steps more are counted
+    launches_per_step, kernels = 1, None
+    if d.q == 9:
+        launches, kernels = counted_launches(torch, lat, args.steps)
+        launches_per_step = launches / args.steps
     bytes_cell = algorithmic_bytes_per_cell(d)
     value = world * N * args.steps / el / 1e6
     avg_launch_s = el / (args.steps * launches_per_step)
@@ -884,16 +895,15 @@ def run_ours(args, rank, world, local_rank):
                    "bytes_per_cell_update": bytes_cell,
                    "l2": f"inputs larger than L2: {N * d.q * storage_bytes(head_storage) / 1e9:.2f} GB per population buffer"
                    if N * d.q * storage_bytes(head_storage) > 126e6 else
-                   ("lattice resident in one thread-block cluster's shared memory for up to 4096 steps per launch"
-                    if kernel_family == "cluster" else "lattice is L2-resident (no flush)"),
+                   ("lattice is L2-resident (no flush); several steps per launch in shared memory"
+                    if launches_per_step < 1 else "lattice is L2-resident (no flush)"),
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
                    "kernel_family": kernel_family, "block": block_used},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"
                      if peak_kind == "measured" else "fallback 6.65 TB/s",
-                     "kernel": ("k_step_sc_window" if d.collision == 2 else "k_step_rows") if kernel_family == "rows"
-                     else "k_step_cluster" if kernel_family == "cluster"
-                     else {0: "k_step_bgk", 1: "k_step_mrt", 2: "k_step_sc + k_sc_psi"}[d.collision],
+                     "kernel": " + ".join(kernels) if kernels else "k_step_rows" if kernel_family == "rows"
+                     else {0: "k_step_bgk", 1: "k_step_mrt"}[d.collision],
                      "bytes_per_launch": bytes_cell * N / launches_per_step},
         "gpu_launches": round(args.steps * launches_per_step),
         "clocks": clocks,
