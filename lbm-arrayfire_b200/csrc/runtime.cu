@@ -677,16 +677,14 @@ static cudaError_t launch_tiles(lbm_ctx* c, int from, cudaStream_t s, int T) {
 }
 
 // The plan, and whether its tiles can run in rounds: what they exchange is allocated with the lattice, or at the first
-// run that is long enough (members of an ensemble, which the ensemble steps).  Not in a capture, nor where memory is
-// out: then one launch a round.
+// run (members of an ensemble, which the ensemble steps).  Where memory is out: one launch a round.
 static bool tiles_ready(lbm_ctx* c) {
     if (!c->sms && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->d.device) != cudaSuccess) return false;
     c->tiles = plan_tiles(c->d, c->sms);
     TileExchange& e = c->tile_ex;
     if (e.records) return true;
     e = tile_exchange(c->d, c->tiles);
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (!e.bytes || cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+    if (!e.bytes) return false;
     const size_t all = e.bytes + sizeof(unsigned) * c->sms;
     if (cudaMalloc(&e.records, all) != cudaSuccess || cudaMemsetAsync(e.records, 0, all, c->stream) != cudaSuccess) {
         cudaGetLastError();
@@ -1095,12 +1093,24 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
     }
     LBM_CK(cudaEventRecord(c->e0, c->stream));
     long long n = nsteps;
-    if (tiles_apply(c)) {
-        const int most = tiles_ready(c) ? tile_launch_steps(c->tiles) : c->tiles.steps;
+    // (a captured run keeps single steps: it is replayed from the buffer that it was captured from, so an even run has
+    // to leave its state there)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool live = cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (!live) cudaGetLastError();
+    c->tiles = TilePlan{};
+    if (live && tiles_apply(c)) {
+        int most = tiles_ready(c) ? tile_launch_steps(c->tiles) : c->tiles.steps;
         // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
         while (c->tiles.kind != kTilesNone && n > 2) {
             const int k = (int)std::min<long long>((n - 1) / 2 * 2, most);
-            LBM_CK(launch_tiles(c, c->cur, c->stream, k));
+            const cudaError_t e = launch_tiles(c, c->cur, c->stream, k);
+            if (e == cudaErrorCooperativeLaunchTooLarge && k > c->tiles.steps) {  // fewer SMs than the device has
+                cudaGetLastError();
+                most = c->tiles.steps;
+                continue;
+            }
+            LBM_CK(e);
             c->cur ^= 1;
             n -= k;
         }
@@ -1123,7 +1133,7 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
         c->cur ^= 1;
         --n;
     }
-    if (n > 2) {
+    if (n > 2 && (live || c->gsteps)) {  // (in a capture no graph of the engine's own can be captured)
         if (!c->gsteps) {
             int rc = build_graphs(c);
             if (rc) return rc;

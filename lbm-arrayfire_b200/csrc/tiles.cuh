@@ -38,7 +38,7 @@
 // which they sent after reading the last ones.  Waits are bounded (two seconds, then an error).
 //
 // Measured on B200 (us per step, one-step kernels -> one launch per T steps -> rounds, lid cavities): 128^2 FP32 1.74 ->
-// 0.90 -> 0.77 and FP16S 2.07 -> 1.03 -> 0.91 (8 steps of 16 x 8 tiles); 512^2 FP32 4.6 -> 3.3 -> 2.65; 1024 x 256 channel
+// 0.90 -> 0.79 and FP16S 2.07 -> 1.03 -> 0.92 (8 steps of 16 x 8 tiles); 512^2 FP32 4.6 -> 3.3 -> 2.65; 1024 x 256 channel
 // FP32 4.5 -> 3.6 -> 3.0; 1000 x 300 channel FP16S 5.2 -> 4.4 -> 3.8; many tiles a CTA: 4096^2 FP32 188 -> 118 (142
 // GLUPS; at one crossing per step HBM allows 91).
 //
