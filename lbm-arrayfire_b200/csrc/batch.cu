@@ -943,7 +943,7 @@ int lbm_batch_sync(lbm_batch* b) {
     int e = 0;
     LBM_CK(cudaMemcpy(&e, b->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
-        LBM_CK(cudaMemset(b->err, 0, sizeof(int)));
+        LBM_CK(cudaMemsetAsync(b->err, 0, sizeof(int), b->stream));  // before the next launch, whose error it must not take
         return set_error(LBM_ERR_TIMEOUT, "a row-pipeline barrier wait ran out (the step did not complete)");
     }
     return LBM_OK;

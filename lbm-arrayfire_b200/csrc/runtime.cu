@@ -923,9 +923,8 @@ int create_lattice(const lbm_desc* d, lbm_ctx** out, bool member) {
     bool ok = cudaMalloc(&c->f[0], fbytes) == cudaSuccess && cudaMalloc(&c->f[1], fbytes) == cudaSuccess &&
               cudaMalloc(&c->partial, sizeof(Sums) * c->reduce_blocks) == cudaSuccess &&
               cudaMalloc(&c->sums_out, sizeof(Sums)) == cudaSuccess &&
-              cudaMalloc(&c->err, sizeof(int)) == cudaSuccess && cudaMemset(c->err, 0, sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&c->tick, 2 * sizeof(unsigned)) == cudaSuccess &&
-              cudaMemset(c->tick, 0, 2 * sizeof(unsigned)) == cudaSuccess;
+              cudaMalloc(&c->err, sizeof(int)) == cudaSuccess &&
+              cudaMalloc(&c->tick, 2 * sizeof(unsigned)) == cudaSuccess;
     if (ok && d->mask) ok = cudaMalloc(&c->mask, (size_t)c->N) == cudaSuccess;
     if (ok && d->collision == LBM_SHANCHEN)
         ok = cudaMalloc(&c->psi, (size_t)c->N * (d->storage == LBM_F64 ? 8 : 4)) == cudaSuccess;
@@ -940,6 +939,12 @@ int create_lattice(const lbm_desc* d, lbm_ctx** out, bool member) {
         return set_error(LBM_ERR_CUDA, "stream/event creation failed");
     }
     c->stream = c->own;
+    // (cleared in the order of the stream that uses them: a cudaMemset is not ordered with a non-blocking stream)
+    if (cudaMemsetAsync(c->err, 0, sizeof(int), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->tick, 0, 2 * sizeof(unsigned), c->stream) != cudaSuccess) {
+        destroy_ctx(c);
+        return set_error(LBM_ERR_CUDA, "clearing the error word and the step counter failed");
+    }
     if (d->mask) {
         for (long long k = 0; k < c->N; ++k)
             if (d->mask[k] >= d->n_classes) {
@@ -1163,9 +1168,10 @@ int lbm_sync(lbm_ctx* c) {
     int err = 0;
     LBM_CK(cudaMemcpy(&err, c->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) {
-        LBM_CK(cudaMemset(c->err, 0, sizeof(int)));
+        // in stream order: the next run finds both cleared, and its own error is not cleared with this one
+        LBM_CK(cudaMemsetAsync(c->err, 0, sizeof(int), c->stream));
         if (c->tile_ex.records) {  // tiles that gave up are behind the others
-            LBM_CK(cudaMemset(c->tile_ex.records, 0, c->tile_ex.bytes + sizeof(unsigned) * c->sms));
+            LBM_CK(cudaMemsetAsync(c->tile_ex.records, 0, c->tile_ex.bytes + sizeof(unsigned) * c->sms, c->stream));
         }
         return set_error(LBM_ERR_TIMEOUT, "a row-pipeline wait on a shared-memory stage gave up; results are invalid");
     }
