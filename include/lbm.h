@@ -159,7 +159,9 @@ int  lbm_get_populations(lbm_ctx* c, void* dst, int dtype, int memory);
 /* F = feq(rho, u) per cell, the reference's start state (cpp/d2q9_bgk_lid.cpp:100-107).
  * rho: N doubles or NULL (=1); u: dim*N doubles [ux | uy (| uz)] or NULL (=0).  Host pointers. */
 int  lbm_init_equilibrium(lbm_ctx* c, const double* rho, const double* u);
-/* Advance nsteps time steps, asynchronously on the context stream. */
+/* Advance nsteps time steps, asynchronously on the context stream.  In a stream capture (after one step outside
+ * it) a run of an even number of steps leaves its state in the buffer that it was captured from, so it can
+ * be replayed any number of times, and between further runs of an even number of steps. */
 int  lbm_step(lbm_ctx* c, int64_t nsteps);
 /* Wait for the context's stream; returns LBM_ERR_TIMEOUT if a step kernel gave up a bounded wait. */
 int  lbm_sync(lbm_ctx* c);
@@ -179,7 +181,9 @@ int64_t lbm_steps_done(const lbm_ctx* c);
 void* lbm_stream(lbm_ctx* c);
 /* NULL restores the context's own (non-blocking) stream; the legacy default stream is cudaStreamLegacy. */
 int   lbm_set_stream(lbm_ctx* c, void* stream);
-/* Current population buffer on the device (storage type of the descriptor) and its byte size. */
+/* Current population buffer on the device (storage type of the descriptor) and its byte size.  Which of the two
+ * buffers it is after a run follows from the launches of the run, not from the number of its steps: ask after
+ * every run. */
 void* lbm_device_populations(lbm_ctx* c, size_t* bytes);
 int   lbm_get_desc(const lbm_ctx* c, lbm_desc* out);
 /* Faces of the slowest axis (z planes of D3Q27, y rows of D2Q9) for halo exchanges between slabs of

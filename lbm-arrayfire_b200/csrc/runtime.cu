@@ -161,6 +161,7 @@ struct lbm_ctx {
     WaitLimits stall = kProductionWaits;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
     int gsteps = 0;
+    bool captured = false;         // some run of it was captured: runs keep the parity of single steps
     bool has_prev = false;
     long long steps = 0;
     double scale = 1.0;
@@ -1098,18 +1099,33 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
     }
     LBM_CK(cudaEventRecord(c->e0, c->stream));
     long long n = nsteps;
-    // (a captured run keeps single steps: it is replayed from the buffer that it was captured from, so an even run has
-    // to leave its state there)
+    // A captured run is replayed from the buffer that it was captured from, also between live runs: an even run has to
+    // leave its state where it found it, as single steps do.  So a captured run takes no tiles, and from the first
+    // captured run of a lattice on, its launches of several steps, each of which changes the buffer once, are as many as
+    // its steps, modulo two.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     const bool live = cudaStreamIsCapturing(c->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-    if (!live) cudaGetLastError();
+    if (!live) {
+        cudaGetLastError();
+        c->captured = true;
+    }
     c->tiles = TilePlan{};
     if (live && tiles_apply(c)) {
         int most = tiles_ready(c) ? tile_launch_steps(c->tiles) : c->tiles.steps;
         // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
-        while (c->tiles.kind != kTilesNone && n > 2) {
-            const int k = (int)std::min<long long>((n - 1) / 2 * 2, most);
-            const cudaError_t e = launch_tiles(c, c->cur, c->stream, k);
+        long long left = c->tiles.kind == kTilesNone ? 0 : (n - 1) / 2 * 2;
+        int turned = 0;
+        while (left > 0) {
+            long long launches = (left + most - 1) / most, k = std::min<long long>(left, most);
+            if (c->captured && ((turned + launches) & 1)) {
+                if (left / 2 == launches) {  // two steps each: two steps fewer
+                    left -= 2;
+                    continue;
+                }
+                ++launches;
+                k = (left / 2 + launches - 1) / launches * 2;
+            }
+            const cudaError_t e = launch_tiles(c, c->cur, c->stream, (int)k);
             if (e == cudaErrorCooperativeLaunchTooLarge && k > c->tiles.steps) {  // fewer SMs than the device has
                 cudaGetLastError();
                 most = c->tiles.steps;
@@ -1117,12 +1133,16 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
             }
             LBM_CK(e);
             c->cur ^= 1;
+            turned ^= 1;
             n -= k;
+            left -= k;
         }
     }
     if (c->kernel_used == LBM_KERNEL_CLUSTER && c->tiles.kind == kTilesNone) {
-        while (n > 0) {
-            const int k = (int)std::min<long long>(n, kClusterMaxSteps);
+        long long launches = (n + kClusterMaxSteps - 1) / kClusterMaxSteps;
+        if (c->captured && ((launches ^ n) & 1)) ++launches;  // (n >= 2: an odd number of launches of an even run, or n > 4096)
+        for (; launches > 0; --launches) {
+            const int k = c->captured ? (int)((n + launches - 1) / launches) : (int)std::min<long long>(n, kClusterMaxSteps);
             launch_cluster(c, c->cur, c->stream, k);
             c->cur ^= 1;
             n -= k;
@@ -1138,7 +1158,8 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
         c->cur ^= 1;
         --n;
     }
-    if (n > 2 && (live || c->gsteps)) {  // (in a capture no graph of the engine's own can be captured)
+    const bool tiled = c->tiles.kind != kTilesNone;  // (a few single steps are left)
+    if (n > 2 && !tiled && (live || c->gsteps)) {  // (in a capture no graph of the engine's own can be captured)
         if (!c->gsteps) {
             int rc = build_graphs(c);
             if (rc) return rc;
