@@ -232,7 +232,8 @@ int   lbm_get_block(const lbm_ctx* c);
  * inside CUDA graphs take PLAIN.  AUTO (default): the autotuner times the eligible ones; besides, runs of
  * three and more steps of a D2Q9 BGK or Shan-Chen lattice advance several steps per launch, on
  * overlapped tiles in shared memory, where that is faster (BGK lattices that one wave of CTAs covers,
- * which stay there for the whole run; FP32 and FP64 ones beyond L2; most Shan-Chen ones).
+ * which stay there for the whole run; FP32 and FP64 ones beyond L2; most Shan-Chen ones).  Small lattices with runs
+ * under way on several streams, which tiles would run one after another, keep single steps or clusters.
  * All give bit-identical results.                                                                   */
 enum lbm_kernel { LBM_KERNEL_AUTO = 0, LBM_KERNEL_PLAIN = 1, LBM_KERNEL_ROWS = 2, LBM_KERNEL_CLUSTER = 3 };
 int   lbm_set_kernel(lbm_ctx* c, int kind);
@@ -253,6 +254,10 @@ int  lbm_test_stall_next_step(lbm_ctx* c, int64_t item, int64_t wait_clocks);
  * ones on lattices with Q N <= 2^32), so that tests can compare both forms bit for bit on small
  * lattices; on = 0 restores the choice.                                                           */
 int  lbm_test_index64(lbm_ctx* c, int on);
+/* Test hook: the tiles of the last lbm_step: their shape (0: the run took single steps or one cluster, 1: 16
+ * columns, 2: 64 columns, 3: 64 columns moved in pieces, 4: 64 columns streamed, 5: Shan-Chen), rows, steps of a
+ * launch or round, and whether they stayed in their CTAs for several rounds.  Any pointer may be NULL. */
+int  lbm_test_last_tiles(const lbm_ctx* c, int* shape, int* rows, int* steps, int* rounds);
 
 /* ---- conservation sums without allocation -----------------------------------------------
  * No counterpart in the reference.  For callers that cannot let a library call cudaMalloc or

@@ -147,7 +147,8 @@ struct lbm_ctx {
     int rows_grid = 0;             // persistent grid of the row pipeline (a whole step)
     int rows_per_sm = 0, sms = 0;  // its CTAs per SM and the device's SMs
     int reserved_sms = 0;          // lbm_set_reserved_sms: SMs the persistent grids leave free
-    TilePlan tiles;                // several steps per launch (tiles.cuh)
+    TilePlan tiles;                // several steps per launch (tiles.cuh), of the last run
+    bool tile_rounds = false;      // the last run had launches in rounds
     bool tune_block = true;        // the block width is left to the autotuner
     int cl_ctas = 0, cl_rows = 0;  // cluster-resident kernel: CTAs of the cluster, rows per CTA
     int rows_rpg = 1;              // its rows per group (segmented rows: the segment width)
@@ -161,6 +162,8 @@ struct lbm_ctx {
     WaitLimits stall = kProductionWaits;
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
     int gsteps = 0;
+    unsigned long long run_no = 0; // its last run's number among all lattices' (begin_run)
+    int beside = 0;                // streams of other lattices with runs beside its last one (begin_run)
     bool captured = false;         // some run of it was captured: runs keep the parity of single steps
     bool has_prev = false;
     long long steps = 0;
@@ -697,6 +700,80 @@ static bool tiles_ready(lbm_ctx* c) {
     return true;
 }
 
+// ---- runs under way on other streams ----------------------------------------------------------
+// Tiles take every SM, so runs on tiles go one after another where single steps (or clusters) of small lattices on
+// streams of their own share the GPU.  Which lattices have runs under way is known on the host alone: lbm_step enters
+// a lattice, every call that waits for its stream takes it out.  It decides between forms with equal results only.
+static std::mutex g_runs_mu;
+// lattices whose last run has not been waited for (never destroyed: a program may destroy lattices at its exit)
+static std::vector<lbm_ctx*>& g_runs = *new std::vector<lbm_ctx*>;
+static unsigned long long g_run_no = 0;
+
+// Enters a run of c.  Returns the number of other streams of the device with runs beside this run or, where a program
+// starts all its lattices and then waits for all, beside the last one.  (Only lattices that were stepped since c was count:
+// one that its program waited for by other means is not waited for here.)
+static int begin_run(lbm_ctx* c) {
+    std::lock_guard<std::mutex> g(g_runs_mu);
+    auto beside = [&](const lbm_ctx* o) {
+        return o != c && o->d.device == c->d.device && o->stream != c->stream && o->run_no > c->run_no;
+    };
+    std::vector<cudaStream_t> streams;
+    for (const lbm_ctx* o : g_runs)
+        if (beside(o) && std::find(streams.begin(), streams.end(), o->stream) == streams.end()) streams.push_back(o->stream);
+    const int now = (int)streams.size(), before = c->beside;
+    for (lbm_ctx* o : g_runs)
+        if (beside(o)) o->beside = std::max(o->beside, now);
+    if (std::find(g_runs.begin(), g_runs.end(), c) == g_runs.end()) g_runs.push_back(c);
+    c->beside = now;
+    c->run_no = ++g_run_no;
+    return std::max(before, now);
+}
+
+static void end_run(lbm_ctx* c) {
+    std::lock_guard<std::mutex> g(g_runs_mu);
+    g_runs.erase(std::remove(g_runs.begin(), g_runs.end(), c), g_runs.end());
+}
+
+// Waits for the lattice's stream.
+static cudaError_t wait_for(lbm_ctx* c) {
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    end_run(c);
+    return e;
+}
+
+// Steps of one of the engine's graphs (even): some 400 us of work.
+static int graph_steps(const lbm_ctx* c) {
+    const double bytes = (double)c->N * c->q * c->sbytes * 2.0;
+    const double est_us = bytes / 5.0e6 + 2.0;  // ~5 TB/s plus launch latency
+    const int g = (int)std::ceil(400.0 / est_us);
+    return std::max(2, std::min(256, g + (g & 1)));
+}
+
+// Whether single steps serve the lattices better with runs on `others` more streams (measured on B200 with K equal lattices,
+// us per lattice and step, single steps or clusters : tiles).
+// - 16-column tiles, 8 steps: 64^2 FP32 K = 2 0.51 : 0.65, K = 8 0.19 : 0.64; 128^2 FP32 K = 2 0.90 : 0.79, K = 3 0.60 : 0.78,
+//   K = 8 0.33 : 0.78, FP64 K = 2 1.12 : 1.26.  4 steps: 192^2 FP32 K = 3 1.14 : 1.05, K = 4 0.86 : 1.04, FP16S K = 3 1.21 :
+//   1.17, K = 4 0.98 : 1.17.
+// - 64-column tiles: 256^2 FP32 K = 2 1.69 : 1.26, K = 3 1.30 : 1.26, K = 8 0.84 : 1.26; 384^2 FP32 K = 2 1.90 : 1.81, K = 3 1.38 :
+//   1.80, FP64 K = 2 2.22 : 3.28; 512^2 FP32 K = 3 2.25 : 2.54, but K = 6, whose buffers leave L2, 2.97 : 2.54; 1000 x 300 FP32
+//   K = 3 2.72 : 2.68, FP16S K = 2 3.12 : 3.33; 640 x 400 FP64 K = 2 3.44 : 4.60, K = 4 5.42 : 4.59.
+// - Shan-Chen: 128^2 FP32 K = 4 1.99 : 1.59, K = 6 1.50 : 1.55, BF16S K = 4 1.52 : 1.70; 256^2 FP32 K = 6 1.61 : 2.09; 512^2 FP32
+//   K = 4 4.35 : 4.67, K = 8 5.47 : 4.95.
+// Lattices of several waves of tiles fill the GPU either way, and short runs of single steps are launched one by one by the
+// host, which tiles spare (runs of 10 steps, K = 4: 256^2 FP32 2.97 : 1.40, but 128^2, a launch a run in a cluster, 0.80 : 1.09).
+static bool gives_way(const lbm_ctx* c, const TilePlan& plan, int others, long long n) {
+    if (!others || (c->kernel_used != LBM_KERNEL_CLUSTER && n < 3 * graph_steps(c))) return false;
+    const int word = c->sbytes;
+    if (plan.kind == kTilesShanChen) return c->N <= 65536 && others >= (word == 2 ? 3 : 5);
+    if (plan.kind == kTilesSmall && plan.steps == 8) return others >= (word == 8 || c->N <= 12288 ? 1 : 2);
+    if (plan.kind == kTilesSmall) return others >= (word == 8 ? 1 : 3);
+    if (plan.kind != kTilesMid) return false;
+    if (c->N <= 200000) return others >= (word == 8 ? 1 : 2);
+    if (word == 2) return true;
+    const bool in_l2 = 2.0 * c->q * word * (double)c->N * (others + 1) <= 112e6;
+    return in_l2 && (word == 8 || (others >= 2 && c->N <= 280000));
+}
+
 static std::mutex g_tune_mu;
 static std::map<std::string, int> g_tune_cache;
 
@@ -818,10 +895,7 @@ static void drop_graphs(lbm_ctx* c) {
 // Capture `gsteps` (even) consecutive steps starting from each buffer parity.
 static int build_graphs(lbm_ctx* c) {
     drop_graphs(c);
-    const double bytes = (double)c->N * c->q * c->sbytes * 2.0;
-    const double est_us = bytes / 5.0e6 + 2.0;  // ~5 TB/s plus launch latency
-    int g = (int)std::ceil(400.0 / est_us);
-    g = std::max(2, std::min(256, g + (g & 1)));
+    const int g = graph_steps(c);
     for (int start = 0; start < 2; ++start) {
         cudaGraph_t graph;
         LBM_CK(cudaStreamBeginCapture(c->own, cudaStreamCaptureModeThreadLocal));
@@ -850,6 +924,7 @@ static int ensure_staging(lbm_ctx* c, size_t bytes) {
 
 static void destroy_ctx(lbm_ctx* c) {
     if (!c) return;
+    end_run(c);
     cudaSetDevice(c->d.device);
     if (c->own) cudaStreamSynchronize(c->own);
     if (c->stream && c->stream != c->own) cudaStreamSynchronize(c->stream);
@@ -1001,7 +1076,7 @@ int lbm_init_equilibrium(lbm_ctx* c, const double* rho, const double* u) {
         });
     });
     LBM_CK(cudaGetLastError());
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     c->has_prev = false;
     return LBM_OK;
 }
@@ -1044,7 +1119,7 @@ int lbm_set_populations(lbm_ctx* c, const void* src, int dtype, int memory) {
             LBM_CK(cudaGetLastError());
         }
     }
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     c->has_prev = false;
     return LBM_OK;
 }
@@ -1084,7 +1159,7 @@ int lbm_get_populations(lbm_ctx* c, void* dst, int dtype, int memory) {
             if (memory == LBM_HOST) LBM_CK(cudaMemcpyAsync(plane, c->staging, elt * c->N, kind, c->stream));
         }
     }
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     return LBM_OK;
 }
 
@@ -1109,9 +1184,12 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
         cudaGetLastError();
         c->captured = true;
     }
+    const int others = live ? begin_run(c) : 0;
     c->tiles = TilePlan{};
+    c->tile_rounds = false;
     if (live && tiles_apply(c)) {
         int most = tiles_ready(c) ? tile_launch_steps(c->tiles) : c->tiles.steps;
+        if (gives_way(c, c->tiles, others, n)) c->tiles = TilePlan{};
         // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
         long long left = c->tiles.kind == kTilesNone ? 0 : (n - 1) / 2 * 2;
         int turned = 0;
@@ -1132,6 +1210,7 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
                 continue;
             }
             LBM_CK(e);
+            c->tile_rounds = c->tile_rounds || k > c->tiles.steps;
             c->cur ^= 1;
             turned ^= 1;
             n -= k;
@@ -1185,7 +1264,7 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
 int lbm_sync(lbm_ctx* c) {
     if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     int err = 0;
     LBM_CK(cudaMemcpy(&err, c->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) {
@@ -1204,6 +1283,7 @@ int lbm_last_step_ms(lbm_ctx* c, float* ms) {
     if (!c->timed) return set_error(LBM_ERR_STATE, "no step has been issued");
     LBM_CK(cudaSetDevice(c->d.device));
     LBM_CK(cudaEventSynchronize(c->e1));
+    end_run(c);
     LBM_CK(cudaEventElapsedTime(ms, c->e0, c->e1));
     return LBM_OK;
 }
@@ -1258,7 +1338,7 @@ int lbm_get_macros(lbm_ctx* c, void* rho, void* u, int dtype, int memory) {
         if (rho) LBM_CK(cudaMemcpyAsync(rho, drho, elt * c->N, cudaMemcpyDeviceToHost, c->stream));
         if (u) LBM_CK(cudaMemcpyAsync(u, du, elt * c->N * c->dim, cudaMemcpyDeviceToHost, c->stream));
     }
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     return LBM_OK;
 }
 
@@ -1277,7 +1357,7 @@ int lbm_sums_fp64(lbm_ctx* c, double out[4]) {
     LBM_CK(cudaGetLastError());
     Sums s;
     LBM_CK(cudaMemcpyAsync(&s, c->sums_out, sizeof(Sums), cudaMemcpyDeviceToHost, c->stream));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     out[0] = s.m;
     out[1] = s.jx;
     out[2] = s.jy;
@@ -1303,7 +1383,7 @@ int lbm_residual_fp64(lbm_ctx* c, double* out) {
     LBM_CK(cudaGetLastError());
     Sums s;
     LBM_CK(cudaMemcpyAsync(&s, c->sums_out, sizeof(Sums), cudaMemcpyDeviceToHost, c->stream));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     *out = s.jx > 0 ? std::sqrt(s.m / s.jx) : 0.0;
     if (!std::isfinite(*out)) return set_error(LBM_ERR_DIVERGED, "residual is not finite");
     return LBM_OK;
@@ -1314,7 +1394,8 @@ void* lbm_stream(lbm_ctx* c) { return c ? (void*)c->stream : nullptr; }
 int lbm_set_stream(lbm_ctx* c, void* stream) {
     if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
+    std::lock_guard<std::mutex> g(g_runs_mu);  // (read by other lattices' begin_run)
     c->stream = stream ? static_cast<cudaStream_t>(stream) : c->own;
     return LBM_OK;
 }
@@ -1350,7 +1431,7 @@ static int face_copy(lbm_ctx* c, int64_t plane, const int32_t* dirs, int32_t ndi
         else
             LBM_CK(cudaMemcpyAsync(dev, io + k * bytes, bytes, kind, c->stream));
     }
-    if (memory == LBM_HOST) LBM_CK(cudaStreamSynchronize(c->stream));
+    if (memory == LBM_HOST) LBM_CK(wait_for(c));
     return LBM_OK;
 }
 
@@ -1373,7 +1454,7 @@ int lbm_set_block(lbm_ctx* c, int threads_x) {
     if (threads_x != 0 && (threads_x < 32 || threads_x > max_block(c) || (threads_x & 31)))
         return set_error(LBM_ERR_INVALID, "block width must be 0 or a multiple of 32 within the kernel's launch bound");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     drop_graphs(c);
     c->block = threads_x;
     c->tune_block = threads_x == 0;
@@ -1399,7 +1480,7 @@ int lbm_set_kernel(lbm_ctx* c, int kind) {
                          "the row pipeline needs D3Q27 BGK/MRT or D2Q9 BGK, deviation arithmetic, F32/F16S/BF16S "
                          "and nx >= 32 a multiple of 16");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     drop_graphs(c);
     c->kernel = kind;
     c->kernel_used = 0;
@@ -1442,7 +1523,7 @@ int lbm_set_reserved_sms(lbm_ctx* c, int sms) {
     if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
     if (sms < 0 || sms > 64) return set_error(LBM_ERR_INVALID, "reserved SMs must be in [0, 64]");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     drop_graphs(c);  // the graphs captured the persistent grid
     c->reserved_sms = sms;
     return LBM_OK;
@@ -1459,7 +1540,7 @@ int lbm_device_buffers(lbm_ctx* c, void** current, void** next, size_t* bytes) {
 int lbm_set_cell_offset(lbm_ctx* c, int64_t offset) {
     if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     drop_graphs(c);  // the graphs captured the old offset in their launch parameters
     c->cell_offset = offset;
     c->pf = make_params<float>(c);
@@ -1483,9 +1564,18 @@ int lbm_test_stall_next_step(lbm_ctx* c, int64_t item, int64_t wait_clocks) {
 int lbm_test_index64(lbm_ctx* c, int on) {
     if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
     LBM_CK(cudaSetDevice(c->d.device));
-    LBM_CK(cudaStreamSynchronize(c->stream));
+    LBM_CK(wait_for(c));
     drop_graphs(c);  // captured launches name the kernel instance
     c->index64 = on != 0;
+    return LBM_OK;
+}
+
+int lbm_test_last_tiles(const lbm_ctx* c, int* shape, int* rows, int* steps, int* rounds) {
+    if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
+    if (shape) *shape = c->tiles.kind;
+    if (rows) *rows = c->tiles.h;
+    if (steps) *steps = c->tiles.steps;
+    if (rounds) *rounds = c->tile_rounds ? 1 : 0;
     return LBM_OK;
 }
 

@@ -128,6 +128,7 @@ _SIGS = {
     "lbm_get_kernel": (C.c_int, [_P]),
     "lbm_test_stall_next_step": (C.c_int, [_P, C.c_int64, C.c_int64]),
     "lbm_test_index64": (C.c_int, [_P, C.c_int]),
+    "lbm_test_last_tiles": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lbm_set_cell_offset": (C.c_int, [_P, C.c_int64]),
     "lbm_step_planes": (C.c_int, [_P, C.c_int64, C.c_int64, C.c_int64, C.c_int, _P]),
     "lbm_set_reserved_sms": (C.c_int, [_P, C.c_int]),
@@ -406,6 +407,12 @@ class Lattice:
         """Test hook: the plain step kernels and the one-pass Shan-Chen kernel index populations in 64
         bits (see lbm_test_index64)."""
         _check(lib().lbm_test_index64(self._h, int(bool(on))))
+
+    def test_last_tiles(self):
+        """Test hook: (shape, rows, steps, rounds) of the last run's tiles (see lbm_test_last_tiles); shape 0: none."""
+        v = [C.c_int() for _ in range(4)]
+        _check(lib().lbm_test_last_tiles(self._h, *(C.byref(a) for a in v)))
+        return tuple(a.value for a in v)
 
     def device_populations(self):
         nbytes = C.c_size_t()
