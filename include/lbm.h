@@ -254,6 +254,9 @@ int  lbm_test_stall_next_step(lbm_ctx* c, int64_t item, int64_t wait_clocks);
  * ones on lattices with Q N <= 2^32), so that tests can compare both forms bit for bit on small
  * lattices; on = 0 restores the choice.                                                           */
 int  lbm_test_index64(lbm_ctx* c, int on);
+/* Test hook: frees what the lattice's tiles exchange, as where lbm_create found no memory for it: the tiles of a
+ * run then take one launch per few steps. */
+int  lbm_test_without_exchange(lbm_ctx* c);
 /* Test hook: the tiles of the last lbm_step: their shape (0: the run took single steps or one cluster, 1: 16
  * columns, 2: 64 columns, 3: 64 columns moved in pieces, 4: 64 columns streamed, 5: Shan-Chen), rows, steps of a
  * launch or round, and whether they stayed in their CTAs for several rounds.  Any pointer may be NULL. */

@@ -147,7 +147,8 @@ struct lbm_ctx {
     int rows_grid = 0;             // persistent grid of the row pipeline (a whole step)
     int rows_per_sm = 0, sms = 0;  // its CTAs per SM and the device's SMs
     int reserved_sms = 0;          // lbm_set_reserved_sms: SMs the persistent grids leave free
-    TilePlan tiles;                // several steps per launch (tiles.cuh), of the last run
+    TilePlan plan;                 // several steps per launch (tiles.cuh)
+    TilePlan tiles;                // what the last run took of it
     bool tile_rounds = false;      // the last run had launches in rounds
     bool tune_block = true;        // the block width is left to the autotuner
     int cl_ctas = 0, cl_rows = 0;  // cluster-resident kernel: CTAs of the cluster, rows per CTA
@@ -680,24 +681,26 @@ static cudaError_t launch_tiles(lbm_ctx* c, int from, cudaStream_t s, int T) {
     return launch_tiles(c->d, l, c->tiles, T, s);
 }
 
-// The plan, and whether its tiles can run in rounds: what they exchange is allocated with the lattice, or at the first
-// run (members of an ensemble, which the ensemble steps).  Where memory is out: one launch a round.
-static bool tiles_ready(lbm_ctx* c) {
-    if (!c->sms && cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->d.device) != cudaSuccess) return false;
-    c->tiles = plan_tiles(c->d, c->sms);
-    TileExchange& e = c->tile_ex;
-    if (e.records) return true;
-    e = tile_exchange(c->d, c->tiles);
-    if (!e.bytes) return false;
+// The plan of a new lattice, and what its tiles exchange in rounds.  Where memory is out: one launch a round, for good
+// (lbm_step allocates nothing: it may run beside another thread's stream capture, which an allocation would end).
+// Members of an ensemble are stepped by the ensemble alone.
+static void plan_lattice(lbm_ctx* c, bool member) {
+    if (!tiles_apply(c)) return;
+    if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->d.device) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    c->plan = plan_tiles(c->d, c->sms);
+    TileExchange e = tile_exchange(c->d, c->plan);
+    if (member || !e.bytes) return;
     const size_t all = e.bytes + sizeof(unsigned) * c->sms;
     if (cudaMalloc(&e.records, all) != cudaSuccess || cudaMemsetAsync(e.records, 0, all, c->stream) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(e.records);
-        e = TileExchange{};
-        return false;
+        return;
     }
     e.rounds = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(e.records) + e.bytes);
-    return true;
+    c->tile_ex = e;
 }
 
 // ---- runs under way on other streams ----------------------------------------------------------
@@ -1035,7 +1038,7 @@ int create_lattice(const lbm_desc* d, lbm_ctx** out, bool member) {
     c->mrt2 = mrt2_applies(c->d);
     c->pf = make_params<float>(c);
     c->pd = make_params<double>(c);
-    if (!member && tiles_apply(c)) tiles_ready(c);
+    plan_lattice(c, member);
     rc = lbm_init_equilibrium(c, nullptr, nullptr);
     if (rc) {
         destroy_ctx(c);
@@ -1188,8 +1191,8 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
     c->tiles = TilePlan{};
     c->tile_rounds = false;
     if (live && tiles_apply(c)) {
-        int most = tiles_ready(c) ? tile_launch_steps(c->tiles) : c->tiles.steps;
-        if (gives_way(c, c->tiles, others, n)) c->tiles = TilePlan{};
+        if (!gives_way(c, c->plan, others, n)) c->tiles = c->plan;
+        int most = c->tile_ex.records ? tile_launch_steps(c->tiles) : c->tiles.steps;
         // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
         long long left = c->tiles.kind == kTilesNone ? 0 : (n - 1) / 2 * 2;
         int turned = 0;
@@ -1567,6 +1570,15 @@ int lbm_test_index64(lbm_ctx* c, int on) {
     LBM_CK(wait_for(c));
     drop_graphs(c);  // captured launches name the kernel instance
     c->index64 = on != 0;
+    return LBM_OK;
+}
+
+int lbm_test_without_exchange(lbm_ctx* c) {
+    if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
+    LBM_CK(cudaSetDevice(c->d.device));
+    LBM_CK(wait_for(c));
+    cudaFree(c->tile_ex.records);
+    c->tile_ex = TileExchange{};
     return LBM_OK;
 }
 

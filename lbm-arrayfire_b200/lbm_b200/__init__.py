@@ -128,6 +128,7 @@ _SIGS = {
     "lbm_get_kernel": (C.c_int, [_P]),
     "lbm_test_stall_next_step": (C.c_int, [_P, C.c_int64, C.c_int64]),
     "lbm_test_index64": (C.c_int, [_P, C.c_int]),
+    "lbm_test_without_exchange": (C.c_int, [_P]),
     "lbm_test_last_tiles": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lbm_set_cell_offset": (C.c_int, [_P, C.c_int64]),
     "lbm_step_planes": (C.c_int, [_P, C.c_int64, C.c_int64, C.c_int64, C.c_int, _P]),
@@ -407,6 +408,10 @@ class Lattice:
         """Test hook: the plain step kernels and the one-pass Shan-Chen kernel index populations in 64
         bits (see lbm_test_index64)."""
         _check(lib().lbm_test_index64(self._h, int(bool(on))))
+
+    def test_without_exchange(self):
+        """Test hook: frees what the lattice's tiles exchange (see lbm_test_without_exchange)."""
+        _check(lib().lbm_test_without_exchange(self._h))
 
     def test_last_tiles(self):
         """Test hook: (shape, rows, steps, rounds) of the last run's tiles (see lbm_test_last_tiles); shape 0: none."""
