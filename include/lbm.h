@@ -249,6 +249,11 @@ int   lbm_get_kernel(const lbm_ctx* c);              /* the family in use (PLAIN
  * once (it clears the error word).  The populations written by that step are invalid: set or
  * re-initialise them before stepping on.  Needs lbm_set_kernel(c, LBM_KERNEL_ROWS) (BGK or MRT).   */
 int  lbm_test_stall_next_step(lbm_ctx* c, int64_t item, int64_t wait_clocks);
+/* The same for tiles that exchange records (lattices that one wave of tiles covers): sets the round counter of tile
+ * `tile` apart, so that in the next run in rounds neither its neighbours nor it find the records they wait for.  They
+ * give up after the waits' limit (2^32 SM clocks, some two seconds), the other tiles after them; the launch returns,
+ * and lbm_sync reports LBM_ERR_TIMEOUT once and clears what the tiles exchange. */
+int  lbm_test_stall_tiles(lbm_ctx* c, int64_t tile);
 /* Test hook (no counterpart in the reference): on = 1 makes the plain step kernels and the one-pass
  * Shan-Chen kernel index populations in 64 bits even where 32-bit indices suffice (they take 32-bit
  * ones on lattices with Q N <= 2^32), so that tests can compare both forms bit for bit on small

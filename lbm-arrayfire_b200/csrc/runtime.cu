@@ -1276,7 +1276,9 @@ int lbm_sync(lbm_ctx* c) {
         if (c->tile_ex.records) {  // tiles that gave up are behind the others
             LBM_CK(cudaMemsetAsync(c->tile_ex.records, 0, c->tile_ex.bytes + sizeof(unsigned) * c->sms, c->stream));
         }
-        return set_error(LBM_ERR_TIMEOUT, "a row-pipeline wait on a shared-memory stage gave up; results are invalid");
+        return set_error(LBM_ERR_TIMEOUT,
+                         err == kTilesTimeout ? "a tile's wait for its region or for its neighbours' records gave up; results are invalid"
+                                              : "a row-pipeline wait on a shared-memory stage gave up; results are invalid");
     }
     return LBM_OK;
 }
@@ -1561,6 +1563,15 @@ int lbm_test_stall_next_step(lbm_ctx* c, int64_t item, int64_t wait_clocks) {
                          "the stall applies to the row pipeline's bulk-copy stages: pin LBM_KERNEL_ROWS (BGK/MRT) first");
     c->stall = WaitLimits{(unsigned)item, (long long)wait_clocks};
     c->stall_armed = true;
+    return LBM_OK;
+}
+
+int lbm_test_stall_tiles(lbm_ctx* c, int64_t tile) {
+    if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
+    if (!c->tile_ex.records) return set_error(LBM_ERR_STATE, "the lattice has no tiles that exchange records");
+    if (tile < 0 || tile >= c->sms) return set_error(LBM_ERR_INVALID, "tile out of range");
+    LBM_CK(cudaSetDevice(c->d.device));
+    LBM_CK(cudaMemsetAsync(c->tile_ex.rounds + tile, 0x40, sizeof(unsigned), c->stream));  // (even: the slots stay the same)
     return LBM_OK;
 }
 

@@ -334,6 +334,8 @@ struct TileLaunch {
     TileExchange ex;
     int sms;
 };
+// Error word of a tile launch that gave up a wait.
+constexpr int kTilesTimeout = 2;
 // The plan of a D2Q9 BGK or Shan-Chen lattice on a device of `sms` SMs (kTilesNone: single steps are faster).
 TilePlan plan_tiles(const lbm_desc& d, int sms);
 // Most steps of one launch (where plan.steps is less: in rounds).
@@ -601,7 +603,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                 const int b = turn & 1;
                 const bool ok = mbar_wait_bounded(&done[b], (uint32_t)((turn >> 1) & 1));
                 if (vote(2, MT, !ok)) {
-                    if (!ok) atomicExch(err, kRowPipeTimeout);
+                    if (!ok) atomicExch(err, kTilesTimeout);
                     break;
                 }
                 move_out(n, b);
@@ -645,7 +647,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
         uint32_t kind = 0;  // marks among the region's cells
         if constexpr (kMove) {
             const bool ok = mbar_wait_bounded(&full[b], (uint32_t)((turn >> 1) & 1));
-            if (!ok) atomicExch(err, kRowPipeTimeout);
+            if (!ok) atomicExch(err, kTilesTimeout);
             if (any(!ok)) return;
         } else {
             if (classes) {
@@ -1016,7 +1018,7 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                         at[i * PLANE] = S(__hiloint2double((int)wd[2 * i + 1], (int)wd[2 * i]));
                 });
             });
-            if (late) atomicExch(err, kRowPipeTimeout);
+            if (late) atomicExch(err, kTilesTimeout);
             if (any(late)) return;
         }
         if (!kMove && total > T && tid == 0) ex.rounds[n] = base + (unsigned)r;

@@ -127,6 +127,7 @@ _SIGS = {
     "lbm_set_kernel": (C.c_int, [_P, C.c_int]),
     "lbm_get_kernel": (C.c_int, [_P]),
     "lbm_test_stall_next_step": (C.c_int, [_P, C.c_int64, C.c_int64]),
+    "lbm_test_stall_tiles": (C.c_int, [_P, C.c_int64]),
     "lbm_test_index64": (C.c_int, [_P, C.c_int]),
     "lbm_test_without_exchange": (C.c_int, [_P]),
     "lbm_test_last_tiles": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
@@ -403,6 +404,11 @@ class Lattice:
         """Test hook: the next step's row pipeline leaves work item `item` unfilled and gives its waits
         `wait_clocks` clocks; lbm_sync then reports LBM_ERR_TIMEOUT (see lbm_test_stall_next_step)."""
         _check(lib().lbm_test_stall_next_step(self._h, item, wait_clocks))
+
+    def test_stall_tiles(self, tile: int = 0):
+        """Test hook: in the next run in rounds, tile `tile` and its neighbours wait for records in vain, some two seconds
+        (see lbm_test_stall_tiles)."""
+        _check(lib().lbm_test_stall_tiles(self._h, tile))
 
     def test_index64(self, on: bool = True):
         """Test hook: the plain step kernels and the one-pass Shan-Chen kernel index populations in 64

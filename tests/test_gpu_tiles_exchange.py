@@ -32,3 +32,39 @@ def test_without_memory_for_the_exchange(nx, ny, storage):
             assert shape in (1, 2) and rounds == 0
         ref.step(31 + 3 + 9 + 10 + 31)
         assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
+
+
+TIMEOUT = -8
+
+
+@pytest.mark.parametrize("nx,ny,storage,tile", [(128, 128, lb.F32, 77), (180, 164, lb.F16S, 0), (301, 199, lb.F64, 3)])
+def test_tiles_that_wait_in_vain_report_a_timeout(nx, ny, storage, tile):
+    """A tile's neighbours and it give up after two seconds, then theirs; the next run is a clean one."""
+    with lattice(nx, ny, storage) as lat, lattice(nx, ny, storage, lb.KERNEL_PLAIN) as ref:
+        F = lat.get_populations(np.float64)
+        lat.step(30)  # (chooses the family of the single steps)
+        assert lb.lib().lbm_sync(lat._h) == 0
+        lat.test_stall_tiles(tile)
+        lat.step(30)
+        assert lat.test_last_tiles()[3] == 1
+        assert lb.lib().lbm_sync(lat._h) == TIMEOUT
+        assert b"neighbours' records" in lb.lib().lbm_last_error()
+        assert lb.lib().lbm_sync(lat._h) == 0  # reported once
+        ref.step(60)  # (the random words go by the step's number)
+        for other in (lat, ref):
+            other.set_populations(F)
+        for n in (30, 31, 5):
+            lat.step(n)
+            assert lb.lib().lbm_sync(lat._h) == 0
+            ref.step(n)
+            assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
+
+
+def test_the_stall_needs_tiles_that_exchange():
+    with lb.Lattice(lb.make_desc(lb.D3Q27, lb.BGK, lb.F32, (32, 32, 32))) as lat:
+        with pytest.raises(lb.LbmError):
+            lat.test_stall_tiles(0)
+    with lattice(128, 128, lb.F32) as lat:
+        for tile in (-1, 100000):
+            with pytest.raises(lb.LbmError):
+                lat.test_stall_tiles(tile)
