@@ -604,6 +604,10 @@ __global__ void __launch_bounds__(Sh::BLOCK, 1)
                 const bool ok = mbar_wait_bounded(&done[b], (uint32_t)((turn >> 1) & 1));
                 if (vote(2, MT, !ok)) {
                     if (!ok) atomicExch(err, kTilesTimeout);
+                    if constexpr (kBulk) {  // wait, briefly and bounded, for copies that may still land in this CTA's regions
+                        mbar_wait_bounded(&full[b], (uint32_t)((turn >> 1) & 1), 1LL << 28);
+                        if (n + stride < tiles) mbar_wait_bounded(&full[b ^ 1], (uint32_t)(((turn + 1) >> 1) & 1), 1LL << 28);
+                    }
                     break;
                 }
                 move_out(n, b);

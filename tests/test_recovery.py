@@ -22,6 +22,15 @@ def test_clears_are_ordered_with_the_steps():
     assert "cudaMemsetAsync(b->err" in body and not re.findall(r"\bcudaMemset\(", body)
 
 
+def test_movers_that_give_up_wait_for_their_copies():
+    """Bulk copies under way land in shared memory: the warps that issued them may not leave the CTA before, also when a
+    wait gave up."""
+    text = (ROOT / "lbm-arrayfire_b200" / "csrc" / "tiles.cuh").read_text()
+    gives_up = text[text.index("if (vote(2, MT, !ok)) {"):]
+    gives_up = gives_up[:gives_up.index("break;")]
+    assert gives_up.count("mbar_wait_bounded(&full[") == 2  # the tile at hand and the next one
+
+
 @pytest.mark.gpu
 def test_every_stalled_run_reports_its_own_timeout():
     d, m, F0 = cavity3d(n=(64, 48, 40), u_lid=0.1, omega=1.3)
