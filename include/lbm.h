@@ -259,6 +259,10 @@ int  lbm_test_stall_tiles(lbm_ctx* c, int64_t tile);
  * ones on lattices with Q N <= 2^32), so that tests can compare both forms bit for bit on small
  * lattices; on = 0 restores the choice.                                                           */
 int  lbm_test_index64(lbm_ctx* c, int on);
+/* Test hook: counts the floats with bit patterns first .. first + count - 1, and their negatives, whose reciprocal as the
+ * tiles' packed arithmetic forms it differs from the division 1 / a (on the current device; none from 2^-24 up
+ * to 2^126). */
+int  lbm_test_reciprocal(uint32_t first, int64_t count, int64_t* differ);
 /* Test hook: frees what the lattice's tiles exchange, as where lbm_create found no memory for it: the tiles of a
  * run then take one launch per few steps. */
 int  lbm_test_without_exchange(lbm_ctx* c);

@@ -198,4 +198,35 @@ TilePlan plan_tiles(const lbm_desc& d, int sms) {
     return TilePlan{};
 }
 
+// Counts the floats of bit patterns [first, first + count), and their negatives, whose packed reciprocal is not 1 / a.
+__global__ void k_test_reciprocal(uint32_t first, uint64_t count, float one, unsigned long long* differ) {
+    unsigned long long n = 0;
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < count; k += (uint64_t)gridDim.x * blockDim.x) {
+        const float a = __uint_as_float(first + (uint32_t)k);
+        float lo, hi;
+        unpack2(reciprocal(pack2(a, -a), pack2(-a, a)), lo, hi);
+        n += (__float_as_uint(lo) != __float_as_uint(one / a)) + (__float_as_uint(hi) != __float_as_uint(one / -a));
+    }
+    if (n) atomicAdd(differ, n);
+}
+
 }  // namespace lbm
+
+extern "C" int lbm_test_reciprocal(uint32_t first, int64_t count, int64_t* differ) {
+    using namespace lbm;
+    if (!differ) return set_error(LBM_ERR_INVALID, "NULL argument");
+    if (count < 0 || count > (1LL << 32) - (int64_t)first) return set_error(LBM_ERR_INVALID, "bit patterns beyond 2^32");
+    unsigned long long* n = nullptr;
+    unsigned long long got = 0;
+    LBM_CK(cudaMalloc(&n, sizeof(*n)));
+    cudaError_t e = cudaMemset(n, 0, sizeof(*n));
+    if (e == cudaSuccess) {
+        k_test_reciprocal<<<1184, 256>>>(first, (uint64_t)count, 1.0f, n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(&got, n, sizeof(got), cudaMemcpyDeviceToHost);
+    cudaFree(n);
+    LBM_CK(e);
+    *differ = (int64_t)got;
+    return LBM_OK;
+}

@@ -94,7 +94,8 @@ __device__ __forceinline__ float rcp_approx(float a) {
 }
 
 // 1 / a: the hardware's approximation and one Newton step in the form that rounds correctly (Markstein
-// 1990).  Equal to the division for every float with 2^-24 <= |a| < 2^126 (tested on all of them); NaN for
+// 1990).  Equal to the division for every float with 2^-24 <= |a| < 2^126 (lbm_test_reciprocal, over all of them): a
+// density 1 + drho is zero or no less than 2^-24, and above 2^126 the equilibrium's 4.5 rho overflows in either form.  NaN for
 // zero and infinite a, where a velocity j / rho is NaN either way.
 __device__ __forceinline__ f32x2 reciprocal(f32x2 a, f32x2 neg_a) {
     float lo, hi;

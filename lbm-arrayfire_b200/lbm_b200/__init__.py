@@ -129,6 +129,7 @@ _SIGS = {
     "lbm_test_stall_next_step": (C.c_int, [_P, C.c_int64, C.c_int64]),
     "lbm_test_stall_tiles": (C.c_int, [_P, C.c_int64]),
     "lbm_test_index64": (C.c_int, [_P, C.c_int]),
+    "lbm_test_reciprocal": (C.c_int, [C.c_uint32, C.c_int64, C.POINTER(C.c_int64)]),
     "lbm_test_without_exchange": (C.c_int, [_P]),
     "lbm_test_last_tiles": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lbm_set_cell_offset": (C.c_int, [_P, C.c_int64]),
