@@ -1241,7 +1241,7 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
         --n;
     }
     const bool tiled = c->tiles.kind != kTilesNone;  // (a few single steps are left)
-    if (n > 2 && !tiled && (live || c->gsteps)) {  // (in a capture no graph of the engine's own can be captured)
+    if (n > 2 && !tiled && live) {  // (a capture can neither build nor launch a graph of the engine's own)
         if (!c->gsteps) {
             int rc = build_graphs(c);
             if (rc) return rc;

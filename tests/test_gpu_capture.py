@@ -86,3 +86,39 @@ def test_long_captured_and_live_runs_in_one_cluster():
         ref.step(2 + 3 * 4100 + 10000)
         assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
         del graph
+
+
+@pytest.mark.parametrize("built", [False, True])
+@pytest.mark.parametrize("lattice_id,shape,storage", [(lb.D2Q9, (150, 97), lb.F16S), (lb.D3Q27, (48, 20, 16), lb.F32)])
+def test_captures_before_and_after_the_engines_own_graphs(lattice_id, shape, storage, built):
+    """Long live runs of single steps replay graphs of the engine's own; a capture may come before or after the first one."""
+    stream = torch.cuda.Stream()
+    d = lb.make_desc(lattice_id, lb.BGK, storage, shape, omega=1.3)
+    n = int(np.prod(shape))
+    w = lb.velocities(lattice_id)[3]
+    F = (np.repeat(w, n) * (1 + 0.02 * np.random.default_rng(n).standard_normal(len(w) * n))).astype(np.float32)
+    with lb.Lattice(d) as lat, lb.Lattice(d) as ref:
+        for a in (lat, ref):
+            a.set_kernel(lb.KERNEL_PLAIN)
+            a.set_populations(F)
+        lat.set_stream(stream)
+        lat.step(700 if built else 2)
+        ref.step(700 if built else 2)
+        lat.sync()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            lat.step(600)
+        for _ in range(2):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        ref.step(1200)
+        torch.cuda.synchronize()
+        assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
+        lat.step(700)
+        ref.step(700)
+        with torch.cuda.stream(stream):
+            graph.replay()
+        ref.step(600)
+        torch.cuda.synchronize()
+        assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
+        del graph
