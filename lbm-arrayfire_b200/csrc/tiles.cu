@@ -14,7 +14,8 @@ namespace lbm {
 // step against 126 in pieces, 2048 x 1024 19.2 against 20.5), pieces where they stay in L2 (1024^2 10.6 against
 // 11.2) and for Shan-Chen's two steps a launch (1024^2 15.1 against 17.5).
 // Mid: 16 warps, whose pairs a step make three full turns with 113 registers a thread (24 warps with 80: two turns, and
-// slower: FP16S 1000 x 300 4.28 -> 4.03, FP32 256^2 1.74 -> 1.61, 1024 x 256 cavity 3.38 -> 3.27).
+// slower: FP16S 1000 x 300 4.28 -> 4.03, FP32 256^2 1.74 -> 1.61, 1024 x 256 cavity 3.38 -> 3.27).  ptxas spills 116 bytes of
+// the FP64 mid shape, 72 of the FP64 stream, 32 of the FP32 streams (80 registers with 24 warps).
 template <class S>
 constexpr int kMidHalo = sizeof(S) == 2 ? 8 : 4;
 template <class S>
@@ -97,7 +98,11 @@ static cudaError_t launch_kind(const StepParams<typename Codec<S>::Real>& p, con
         return launch_one<S, ABS, Sh, kWord>(p, l, plan, steps, s);
     };
     if constexpr (kWord <= 4 && !ABS) {
-        if (plan.kind == kTilesShanChen) return by_piece(ShanChenShape<S>{});
+        if (plan.kind == kTilesShanChen) {
+            if constexpr (kWord == 4) return by_piece(ShanChenShape<S>{});
+            // (16-bit words: plan_tiles asks for whole 16-byte words)
+            return row % 16 == 0 ? launch_one<S, ABS, ShanChenShape<S>, 16>(p, l, plan, steps, s) : cudaErrorInvalidValue;
+        }
     }
     if constexpr (kWord >= 4 && !ABS) {
         if (plan.kind == kTilesStream && row % 16 == 0) return launch_one<S, ABS, StreamShape<S, true>, 16>(p, l, plan, steps, s);
@@ -141,12 +146,12 @@ cudaError_t launch_tiles(const lbm_desc& d, const TileLaunch& l, const TilePlan&
 // - BGK lattices that one wave of CTAs covers, in rounds of T steps: about 2 us a round for the exchange and T short
 //   steps.  Small tiles first, for more CTAs: 96^2 FP32 1.4 -> 0.7, 128^2 1.8 -> 0.8, 192^2 (16-row tiles, 4 steps)
 //   2.5 -> 1.1; then 64-column tiles: 256^2 2.9 -> 1.3, 512^2 4.6 -> 2.6, 1000 x 300 4.3 -> 2.8; FP16S 192^2 2.7 -> 1.2,
-//   512^2 5.2 -> 3.3, 1000 x 300 5.0 -> 3.5; FP64 256^2 3.3 -> 2.2, 384^2 4.0 -> 3.35, 640 x 400 (32 rows) 5.35 -> 4.75.
+//   512^2 5.2 -> 3.3, 1000 x 300 5.0 -> 3.5; FP64 256^2 3.3 -> 2.2, 384^2 4.0 -> 3.35, 640 x 400 (30 rows) 5.1 -> 4.6.
 // - FP32 BGK in L2, several waves: a wave of h-row tiles takes 2.3 (h + 6) / 36 us, a launch 1.4, a single step 1.5
-//   and its cells at 107 G/s, which decides (1024 x 512 6.6 -> 6.2, 1024^2 11.2 -> 10.6; 1500 x 451 8.0 -> 8.7 stays
-//   single).  16-bit words gain nothing there (1024 x 512 FP16S 7.4 -> 7.2, 1024^2 11.4 -> 13.3).
+//   and its cells at 107 G/s, which decides (1024 x 512 6.3 -> 5.6, 1024^2 11.2 -> 9.0; 1500 x 451 7.6 -> 7.0).
+//   16-bit words gain nothing there (1024 x 512 FP16S 7.4 -> 7.2, 1024^2 11.4 -> 13.3).
 // - BGK lattices whose two buffers leave L2: FP32 from about 80 MB (75 MB 11.2 -> 11.9, 86 MB 13.6 -> 11.8, 151 MB
-//   26.3 -> 19.2, 433 MB 70 -> 45; rows that start anywhere move in pieces, from 125 MB: 433 MB 76 -> 63), FP64 with
+//   26.3 -> 19.2, 433 MB 70 -> 45; rows that start anywhere move in pieces, from 125 MB: 433 MB 78 -> 52), FP64 with
 //   rows of whole 16-byte words from 140 MB (151 MB 24.0 -> 22.4, 302 MB 47 -> 39, 865 MB 132 -> 104; in pieces 134 ->
 //   137).  16-bit words cross HBM fast enough in single steps (2048^2 FP16S 39.6 -> 46.6).
 // - Shan-Chen, FP32 of any width and 16-bit words in rows of whole 16-byte words (in 2-byte pieces 2049 x 1537

@@ -22,7 +22,7 @@
 // instruction does two cells' work in one issue slot and two cycles of the FP32 pipe.  A pair takes 109
 // packed instructions, 24-36 shared-memory accesses and some 20 others; a step of a 64 x 34 tile takes 3000 to
 // 3700 cycles where the FP32 pipe alone needs 2350 (scalar arithmetic: 209 instructions per cell, 110 GLUPS at
-// 4096^2 against 142).  The moves: 16-byte cp.async (.cg: past the small L1 that 227 KB of shared memory leave;
+// 4096^2 without walls against 146).  The moves: 16-byte cp.async (.cg: past the small L1 that 227 KB of shared memory leave;
 // .ca took 710 us per 4 steps at 4096^2 against 540) while the lattice has one tile per SM; where SMs take
 // many tiles, four warps of their own move whole rows by bulk copies beside the computing ones (one warp
 // issues a bulk copy every 58 cycles, four keep up).
@@ -38,9 +38,9 @@
 // which they sent after reading the last ones.  Waits are bounded (two seconds, then an error).
 //
 // Measured on B200 (us per step, one-step kernels -> one launch per T steps -> rounds, lid cavities): 128^2 FP32 1.74 ->
-// 0.90 -> 0.79 and FP16S 2.07 -> 1.03 -> 0.92 (8 steps of 16 x 8 tiles); 512^2 FP32 4.6 -> 3.3 -> 2.65; 1024 x 256 channel
-// FP32 4.5 -> 3.6 -> 3.0; 1000 x 300 channel FP16S 5.2 -> 4.4 -> 3.8; many tiles a CTA: 4096^2 FP32 188 -> 118 (142
-// GLUPS; at one crossing per step HBM allows 91).
+// 0.90 -> 0.78 and FP16S 2.07 -> 1.03 -> 0.91 (8 steps of 16 x 8 tiles); 512^2 FP32 4.2 -> 3.3 -> 2.5; 1024 x 256 channel
+// FP32 3.9 -> 3.6 -> 2.9; 1000 x 300 channel FP16S 5.1 -> 4.4 -> 3.3; many tiles a CTA: 4096^2 FP32 189 -> 120.5 (139
+// GLUPS; without walls 115, 146 GLUPS; at one crossing per step HBM allows 91).
 //
 // The cell update is the other kernels' (bgk_collide, codecs and random words, with the step counter advanced
 // by T), so the results are bit-identical to single steps.  A launch leaves the state after T steps in
