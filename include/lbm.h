@@ -237,7 +237,8 @@ int   lbm_get_block(const lbm_ctx* c);
  * All give bit-identical results.                                                                   */
 enum lbm_kernel { LBM_KERNEL_AUTO = 0, LBM_KERNEL_PLAIN = 1, LBM_KERNEL_ROWS = 2, LBM_KERNEL_CLUSTER = 3 };
 int   lbm_set_kernel(lbm_ctx* c, int kind);
-int   lbm_get_kernel(const lbm_ctx* c);              /* the family in use (PLAIN, ROWS or CLUSTER), or AUTO before the first step */
+int   lbm_get_kernel(const lbm_ctx* c);              /* the family of single steps (PLAIN, ROWS or CLUSTER), which
+                                                      * runs on tiles take for their last; AUTO before the first step */
 
 /* ---- test hook of the bounded device-side waits (no counterpart in the reference) --------
  * Arms a one-shot stall of the row pipeline so that tests can drive its bounded mbarrier waits to

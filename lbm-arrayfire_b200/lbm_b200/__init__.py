@@ -379,6 +379,7 @@ class Lattice:
         _check(lib().lbm_set_kernel(self._h, kind))
 
     def kernel(self) -> int:
+        """The family of single steps, which runs on tiles take for their last (see lbm_get_kernel)."""
         return lib().lbm_get_kernel(self._h)
 
     def step_planes(self, first: int, count: int, finish: bool, stream=None, stride: int = 1):
