@@ -108,6 +108,23 @@ def algorithmic_bytes_per_cell(d):
     return b
 
 
+def crossed_bytes(d, steps, counted):
+    """Bytes of populations that `steps` steps move between HBM or L2 and the SMs, as launched: one read and one write of
+    all of them per step, or, in two dimensions where launches of several steps keep them in shared memory meanwhile,
+    per launch.  counted: the launches (counted_launches), None in three dimensions."""
+    if counted and counted["crossings"] < steps:
+        return 2 * d.q * storage_bytes(d.storage) * d.cells * counted["crossings"]
+    return algorithmic_bytes_per_cell(d) * d.cells * steps
+
+
+def roofline_of(d, steps, seconds, counted, peak):
+    """Achieved GB/s, and what bounds the run: HBM, or, where populations cross it less than once a step, the arithmetic."""
+    achieved = crossed_bytes(d, steps, counted) / seconds / 1e9
+    several = bool(counted) and counted["crossings"] < steps
+    return {"bound": "fp32 pipe and latency (several steps per crossing)" if several else "hbm", "achieved": achieved,
+            "peak": peak, "unit": "GB/s", "frac": achieved / peak}
+
+
 def peaks():
     p = ROOT / "MEASURED_PEAKS.json"
     if p.exists():
@@ -354,6 +371,12 @@ def apply_kernel_choice(lb, lat, args):
 KERNEL_NAMES = {1: "plain", 2: "rows", 3: "cluster"}
 
 
+def family_of(lat):
+    """What the lattice's last run took: tiles (its last step or two singly), or the family of single steps."""
+    family = KERNEL_NAMES.get(lat.kernel(), "unknown")
+    return f"tiles, {family} for single steps" if lat.test_last_tiles()[0] else family
+
+
 def measure(torch, lb, args, storage, dev, world, sample_clocks=False):
     d, m = build_workload(lb, args, storage)
     d.device = dev
@@ -458,7 +481,7 @@ def acc_run(lb, wl, storage, steps, start=None, shape=None, hook=None, nearest=F
         lat.sync()
         rho, u = lat.macros()
         m1 = lat.sums()[0]
-        fam = KERNEL_NAMES.get(lat.kernel(), "unknown")
+        fam = family_of(lat)
     return {"d": d, "m": m, "rho": rho, "u": u, "mass0": m0, "mass1": m1, "family": fam, "extra": extra}
 
 
@@ -494,7 +517,7 @@ def acc_cavity128(lb):
         lat.step(10000)
         rho, u = lat.macros()
         runs["f32_reference_arithmetic"] = {"d": d, "m": m, "rho": rho, "u": u, "mass0": m0,
-                                            "mass1": lat.sums()[0], "family": "plain"}
+                                            "mass1": lat.sums()[0], "family": family_of(lat)}
     out = field_errors(lb, runs, "f64", ["f32", "f16s", "f16s_nearest", "f32_reference_arithmetic"])
     out["steps"] = 10000
     return out
@@ -810,8 +833,8 @@ SMALL_CONFIGS = (("d2q9_lid_128", "f16s", 20000), ("d2q9_channel_1024x256", "f16
 def config_lines(torch, lb, args, dev, world):
     """MLUPS of configs 1-3 (16-bit storage and FP32) and of the config-5 ensemble, each timed like the
     headline (CUDA events on the lattice's stream after warm-up).  Configs 1-3 are L2-resident (their
-    populations fit the 126 MB L2), so no HBM roofline applies to them; their achieved GB/s is stated
-    against the algorithmic bytes."""
+    populations fit the 126 MB L2), so no HBM roofline applies to them; their achieved GB/s is that of the
+    populations that their launches read and write."""
     import copy
 
     out = {}
@@ -822,12 +845,12 @@ def config_lines(torch, lb, args, dev, world):
             a.workload, a.steps, a.warmup = wl, steps, max(args.warmup, 3)
             a.kernel, a.block, a.dims, a.size = "auto", 0, "", 0
             d, lat, el, _ = measure(torch, lb, a, STORAGES[stn], dev, world)
-            launches, kernels = counted_launches(torch, lat, steps)
+            counted = counted_launches(torch, lat, steps)
             lat.close()
             del lat
             rec[stn] = {"value": d.cells * steps / el / 1e6, "unit": "MLUPS", "ms_per_step": el * 1e3 / steps,
-                        "kernels": kernels, "launches_per_step": launches / steps,
-                        "achieved_gbs": algorithmic_bytes_per_cell(d) * d.cells * steps / el / 1e9}
+                        "kernels": counted["kernels"], "launches_per_step": counted["launches"] / steps,
+                        "achieved_gbs": crossed_bytes(d, steps, counted) / el / 1e9}
             rec["lattice"] = list(d.shape)
             mb = d.cells * d.q * storage_bytes(STORAGES[stn]) * 2 / 1e6
             rec["l2"] = (f"L2-resident ({mb:.1f} MB of populations in both buffers at {stn}); no flush; several steps per "
@@ -847,15 +870,24 @@ def config_lines(torch, lb, args, dev, world):
 
 
 def counted_launches(torch, lat, steps):
-    """Kernel launches of `steps` more steps of a lattice, and the kernels' names (outside any timed region)."""
-    import re
-
+    """Kernel launches of `steps` more steps of a lattice, those among them that read and write all populations, and the
+    kernels' names (outside any timed region)."""
     lat.sync()
     with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
         lat.step(steps)
         lat.sync()
-    names = [e.name for e in prof.events() if "k_step" in e.name or "k_sc_psi" in e.name]
-    return len(names), sorted({re.search(r"k_\w+", n).group(0) for n in names})
+    return launch_counts([e.name for e in prof.events()], steps)
+
+
+def launch_counts(names, steps):
+    """The counts from the profiled kernels' names; where the profiler recorded none, one launch a step."""
+    import re
+
+    names = [n for n in names if "k_step" in n or "k_sc_psi" in n]
+    if not names:
+        return {"launches": steps, "crossings": steps, "kernels": ["k_step (not counted)"]}
+    return {"launches": len(names), "crossings": sum("k_step" in n for n in names),
+            "kernels": sorted({re.search(r"k_\w+", n).group(0) for n in names})}
 
 
 def run_ours(args, rank, world, local_rank):
@@ -872,16 +904,13 @@ def run_ours(args, rank, world, local_rank):
     N = d.cells
     # one launch per step, except in two dimensions (several steps per launch on tiles, one per 4096 in a cluster,
     # Shan-Chen's two passes), where the launches of as many steps more are counted
-    launches_per_step, kernels = 1, None
-    if d.q == 9:
-        launches, kernels = counted_launches(torch, lat, args.steps)
-        launches_per_step = launches / args.steps
+    counted = counted_launches(torch, lat, args.steps) if d.q == 9 else None
+    launches = counted["launches"] if counted else args.steps
     bytes_cell = algorithmic_bytes_per_cell(d)
     value = world * N * args.steps / el / 1e6
-    avg_launch_s = el / (args.steps * launches_per_step)
-    achieved = bytes_cell * N / launches_per_step / avg_launch_s / 1e9
+    roofline = roofline_of(d, args.steps, el, counted, peak)
     traffic = dram_traffic(args.workload, head_storage)
-    kernel_family = KERNEL_NAMES.get(lat.kernel(), "unknown")
+    kernel_family = family_of(lat)
     block_used = lat.block()
     lat.close()
     del lat
@@ -896,30 +925,28 @@ def run_ours(args, rank, world, local_rank):
                    "l2": f"inputs larger than L2: {N * d.q * storage_bytes(head_storage) / 1e9:.2f} GB per population buffer"
                    if N * d.q * storage_bytes(head_storage) > 126e6 else
                    ("lattice is L2-resident (no flush); several steps per launch in shared memory"
-                    if launches_per_step < 1 else "lattice is L2-resident (no flush)"),
+                    if launches < args.steps else "lattice is L2-resident (no flush)"),
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
                    "kernel_family": kernel_family, "block": block_used},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": traffic, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"
+        "roofline": {**roofline, "traffic": traffic, "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"
                      if peak_kind == "measured" else "fallback 6.65 TB/s",
-                     "kernel": " + ".join(kernels) if kernels else "k_step_rows" if kernel_family == "rows"
+                     "kernel": " + ".join(counted["kernels"]) if counted else "k_step_rows" if kernel_family == "rows"
                      else {0: "k_step_bgk", 1: "k_step_mrt"}[d.collision],
-                     "bytes_per_launch": bytes_cell * N / launches_per_step},
-        "gpu_launches": round(args.steps * launches_per_step),
+                     "bytes_per_launch": crossed_bytes(d, args.steps, counted) / launches},
+        "gpu_launches": launches,
         "clocks": clocks,
     }
     # FP32 plain beside the 16-bit headline
     if head_storage != lb.F32 and not args.no_compare:
         d32, lat32, el32, clocks32 = measure(torch, lb, args, lb.F32, dev, world, sample_clocks=(rank == 0))
-        family32 = KERNEL_NAMES.get(lat32.kernel(), "unknown")
+        family32 = family_of(lat32)
+        counted32 = counted_launches(torch, lat32, args.steps) if d32.q == 9 else None
         lat32.close()
         del lat32
         v32 = world * N * args.steps / el32 / 1e6
-        b32 = algorithmic_bytes_per_cell(d32)
-        a32 = b32 * N / launches_per_step / (el32 / (args.steps * launches_per_step)) / 1e9
         out["fp32_plain"] = {"value": v32, "unit": "MLUPS", "ms_per_step": el32 * 1e3 / args.steps,
                              "kernel_family": family32, "clocks": clocks32,
-                             "roofline": {"achieved": a32, "peak": peak, "frac": a32 / peak,
+                             "roofline": {**roofline_of(d32, args.steps, el32, counted32, peak),
                                           "traffic": dram_traffic(args.workload, lb.F32)}}
         out[f"speedup_{STORAGE_NAMES[head_storage]}_vs_f32"] = value / v32
     if not args.no_e2e:
