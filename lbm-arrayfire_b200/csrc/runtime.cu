@@ -710,23 +710,30 @@ static void plan_lattice(lbm_ctx* c, bool member) {
 static std::mutex g_runs_mu;
 // lattices whose last run has not been waited for (never destroyed: a program may destroy lattices at its exit)
 static std::vector<lbm_ctx*>& g_runs = *new std::vector<lbm_ctx*>;
+static size_t g_lattices = 0;
 static unsigned long long g_run_no = 0;
 
 // Enters a run of c.  Returns the number of other streams of the device with runs beside this run or, where a program
 // starts all its lattices and then waits for all, beside the last one.  (Only lattices that were stepped since c was count:
-// one that its program waited for by other means is not waited for here.)
+// one that its program waited for by other means is not waited for here.)  The latest runs are last; of very many, the last
+// 32 are looked at.  No allocation here: g_runs has room for every lattice.
 static int begin_run(lbm_ctx* c) {
     std::lock_guard<std::mutex> g(g_runs_mu);
+    const int n = (int)g_runs.size(), from = std::max(0, n - 32);
     auto beside = [&](const lbm_ctx* o) {
         return o != c && o->d.device == c->d.device && o->stream != c->stream && o->run_no > c->run_no;
     };
-    std::vector<cudaStream_t> streams;
-    for (const lbm_ctx* o : g_runs)
-        if (beside(o) && std::find(streams.begin(), streams.end(), o->stream) == streams.end()) streams.push_back(o->stream);
-    const int now = (int)streams.size(), before = c->beside;
-    for (lbm_ctx* o : g_runs)
-        if (beside(o)) o->beside = std::max(o->beside, now);
-    if (std::find(g_runs.begin(), g_runs.end(), c) == g_runs.end()) g_runs.push_back(c);
+    int now = 0;
+    for (int k = from; k < n; ++k) {
+        bool first = beside(g_runs[k]);
+        for (int j = from; first && j < k; ++j) first = !beside(g_runs[j]) || g_runs[j]->stream != g_runs[k]->stream;
+        now += first;
+    }
+    for (int k = from; k < n; ++k)
+        if (beside(g_runs[k])) g_runs[k]->beside = std::max(g_runs[k]->beside, now);
+    const int before = c->beside;
+    g_runs.erase(std::remove(g_runs.begin(), g_runs.end(), c), g_runs.end());
+    g_runs.push_back(c);
     c->beside = now;
     c->run_no = ++g_run_no;
     return std::max(before, now);
@@ -928,6 +935,10 @@ static int ensure_staging(lbm_ctx* c, size_t bytes) {
 static void destroy_ctx(lbm_ctx* c) {
     if (!c) return;
     end_run(c);
+    {
+        std::lock_guard<std::mutex> g(g_runs_mu);
+        --g_lattices;
+    }
     cudaSetDevice(c->d.device);
     if (c->own) cudaStreamSynchronize(c->own);
     if (c->stream && c->stream != c->own) cudaStreamSynchronize(c->stream);
@@ -990,6 +1001,10 @@ int create_lattice(const lbm_desc* d, lbm_ctx** out, bool member) {
     if ((rc = check_device(d->device))) return rc;
     LBM_CK(cudaSetDevice(d->device));
     lbm_ctx* c = new lbm_ctx();
+    {
+        std::lock_guard<std::mutex> g(g_runs_mu);
+        if (g_runs.capacity() < ++g_lattices) g_runs.reserve(2 * g_lattices);
+    }
     c->d = *d;
     c->d.mask = nullptr;
     c->q = desc_q(d);

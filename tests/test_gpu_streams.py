@@ -140,3 +140,16 @@ def test_lattices_on_threads_of_their_own():
     assert not errors
     for k, s in enumerate(sizes):
         assert np.array_equal(out[k], plain(k, *s, 330))
+
+
+def test_hundreds_of_lattices_under_way():
+    """The last 32 runs are looked at: a step call costs the host the same beside hundreds of lattices as beside a few."""
+    lats = [lattice(k, 64, 48) for k in range(200)]
+    for _ in range(2):
+        for lat in lats:
+            lat.step(7)
+    assert shape(lats[0]) == shape(lats[-1]) == 0
+    for k in (0, 99, 199):
+        assert np.array_equal(lats[k].get_populations(np.float64), plain(k, 64, 48, 14))
+    for lat in lats:
+        lat.close()
