@@ -784,6 +784,24 @@ static bool gives_way(const lbm_ctx* c, const TilePlan& plan, int others, long l
     return in_l2 && (word == 8 || (others >= 2 && c->N <= 280000));
 }
 
+// Whether single steps, or one cluster, take less time for a run of n steps than its tiles and the single steps after them
+// (measured on B200, us per run, single steps or cluster : tiles).
+// - A cluster starts in one launch; tiles save steps of 0.3 to 1 us: 64^2 FP32 n = 4 15 : 19, n = 12 22 : 26, n = 24 34 : 33, FP64
+//   n = 32 46 : 50; 80^2 FP32 n = 8 20 : 22, n = 16 30 : 28; 96^2 n = 4 16 : 19, n = 10 24 : 23; 128^2 n = 4 20 : 20, n = 10 28 : 23.
+// - Two steps on tiles move as much as two single ones, and more with their halos: 1200 x 1000 FP32 n = 4 65 : 75, n = 5
+//   81 : 72; 4096^2 FP32 n = 3 571 : 620, n = 5 974 : 679; 640 x 400 FP64 n = 4 34 : 39, n = 5 41 : 39; 1001 x 301 FP16S n = 3
+//   24 : 26; but 256^2 FP32 n = 3 18 : 16, 400^2 FP32 n = 4 30 : 27, and two steps a launch are Shan-Chen's rule.
+static bool too_short(const lbm_ctx* c, const TilePlan& plan, long long n) {
+    const int word = c->sbytes;
+    if (c->kernel_used == LBM_KERNEL_CLUSTER) {
+        if (c->N <= 5000) return n < (word == 8 ? 64 : 24);
+        if (c->N <= 8000) return n < (word == 8 ? 20 : 14);
+        return n == 4 && c->N < 16000;
+    }
+    if (n > 4 || plan.kind == kTilesSmall || plan.kind == kTilesShanChen) return false;
+    return plan.kind != kTilesMid || word == 8 || (word == 2 && c->d.nx % 8) || c->N > 280000;
+}
+
 static std::mutex g_tune_mu;
 static std::map<std::string, int> g_tune_cache;
 
@@ -1206,7 +1224,7 @@ int lbm_step(lbm_ctx* c, int64_t nsteps) {
     c->tiles = TilePlan{};
     c->tile_rounds = false;
     if (live && tiles_apply(c)) {
-        if (!gives_way(c, c->plan, others, n)) c->tiles = c->plan;
+        if (!too_short(c, c->plan, n) && !gives_way(c, c->plan, others, n)) c->tiles = c->plan;
         int most = c->tile_ex.records ? tile_launch_steps(c->tiles) : c->tiles.steps;
         // the last step is a single one: the buffer it reads is the state before it (lbm_get_macros)
         long long left = c->tiles.kind == kTilesNone ? 0 : (n - 1) / 2 * 2;

@@ -26,11 +26,11 @@ def test_without_memory_for_the_exchange(nx, ny, storage):
         lat.step(31)
         assert lat.test_last_tiles()[3] == 1
         lat.test_without_exchange()
-        for n in (3, 9, 10, 31):
+        for n in (5, 9, 10, 31):
             lat.step(n)
             shape, _, _, rounds = lat.test_last_tiles()
             assert shape in (1, 2) and rounds == 0
-        ref.step(31 + 3 + 9 + 10 + 31)
+        ref.step(31 + 5 + 9 + 10 + 31)
         assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
 
 

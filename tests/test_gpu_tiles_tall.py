@@ -72,3 +72,25 @@ def test_runs_beyond_one_launch(kind, nx, ny, shape, rows, steps, storage):
 ])
 def test_many_tiles_a_cta(kind, nx, ny, storage, shape, rows, steps):
     same_as_plain(kind, nx, ny, storage, (7, 18), shape, rows, steps, 0)
+
+
+@pytest.mark.parametrize("kind,nx,ny,storage,few,enough", [
+    ("lid", 64, 64, lb.F32, (3, 10, 23), 24),        # one cluster
+    ("lid", 48, 40, lb.F64, (4, 63), 64),
+    ("lid", 80, 80, lb.F16S, (4, 13), 14),
+    ("lid", 100, 100, lb.F32, (4,), 10),
+    (1, 1200, 1000, lb.F32, (3, 4), 5),              # single steps
+    (1, 641, 401, lb.F64, (3, 4), 5),
+    (0, 1001, 300, lb.F16S, (3, 4), 5),
+    ("lid", 1501, 1201, lb.F32, (3, 4), 5),
+])
+def test_runs_too_short_for_tiles(kind, nx, ny, storage, few, enough):
+    with lattice(kind, nx, ny, storage) as a, lattice(kind, nx, ny, storage, lb.KERNEL_PLAIN) as b:
+        for n in (*few, enough):
+            a.step(n)
+            a.sync()  # (small lattices with runs beside one another take single steps or clusters anyway)
+            b.step(n)
+            b.sync()
+            if a.kernel() == lb.KERNEL_CLUSTER or a.desc.cells > 16384:
+                assert (a.test_last_tiles()[0] != 0) == (n == enough)
+            assert np.array_equal(a.get_populations(np.float64), b.get_populations(np.float64), equal_nan=True)
