@@ -267,6 +267,9 @@ int  lbm_test_reciprocal(uint32_t first, int64_t count, int64_t* differ);
 /* Test hook: frees what the lattice's tiles exchange, as where lbm_create found no memory for it: the tiles of a
  * run then take one launch per few steps. */
 int  lbm_test_without_exchange(lbm_ctx* c);
+/* Test hook: on = 1 answers the lattice's launches in rounds on the host as the runtime does where their CTAs cannot all be
+ * resident (a program that was given fewer SMs than the device has); on = 0 launches them again. */
+int  lbm_test_refuse_rounds(lbm_ctx* c, int on);
 /* Test hook: the tiles of the last lbm_step: their shape (0: the run took single steps or one cluster, 1: 16
  * columns, 2: 64 columns, 3: 64 columns moved in pieces, 4: 64 columns streamed, 5: Shan-Chen), rows, steps of a
  * launch or round, and whether they stayed in their CTAs for several rounds.  Any pointer may be NULL. */

@@ -154,6 +154,7 @@ extern "C" {
     pub fn lbm_test_index64(c: *mut lbm_ctx, on: c_int) -> c_int;
     pub fn lbm_test_reciprocal(first: u32, count: i64, differ: *mut i64) -> c_int;
     pub fn lbm_test_without_exchange(c: *mut lbm_ctx) -> c_int;
+    pub fn lbm_test_refuse_rounds(c: *mut lbm_ctx, on: c_int) -> c_int;
     pub fn lbm_test_last_tiles(
         c: *const lbm_ctx,
         shape: *mut c_int,

@@ -150,6 +150,7 @@ struct lbm_ctx {
     TilePlan plan;                 // several steps per launch (tiles.cuh)
     TilePlan tiles;                // what the last run took of it
     bool tile_rounds = false;      // the last run had launches in rounds
+    bool refuse_rounds = false;    // lbm_test_refuse_rounds
     bool tune_block = true;        // the block width is left to the autotuner
     int cl_ctas = 0, cl_rows = 0;  // cluster-resident kernel: CTAs of the cluster, rows per CTA
     int rows_rpg = 1;              // its rows per group (segmented rows: the segment width)
@@ -669,6 +670,7 @@ static bool tiles_apply(const lbm_ctx* c) {
 
 // One launch of T steps from buffer `from` into the other one.
 static cudaError_t launch_tiles(lbm_ctx* c, int from, cudaStream_t s, int T) {
+    if (c->refuse_rounds && T > c->tiles.steps) return cudaErrorCooperativeLaunchTooLarge;
     TileLaunch l{};
     l.pf = c->pf;
     l.pd = c->pd;
@@ -1623,6 +1625,12 @@ int lbm_test_without_exchange(lbm_ctx* c) {
     LBM_CK(wait_for(c));
     cudaFree(c->tile_ex.records);
     c->tile_ex = TileExchange{};
+    return LBM_OK;
+}
+
+int lbm_test_refuse_rounds(lbm_ctx* c, int on) {
+    if (!c) return set_error(LBM_ERR_INVALID, "context is NULL");
+    c->refuse_rounds = on != 0;
     return LBM_OK;
 }
 

@@ -131,6 +131,7 @@ _SIGS = {
     "lbm_test_index64": (C.c_int, [_P, C.c_int]),
     "lbm_test_reciprocal": (C.c_int, [C.c_uint32, C.c_int64, C.POINTER(C.c_int64)]),
     "lbm_test_without_exchange": (C.c_int, [_P]),
+    "lbm_test_refuse_rounds": (C.c_int, [_P, C.c_int]),
     "lbm_test_last_tiles": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lbm_set_cell_offset": (C.c_int, [_P, C.c_int64]),
     "lbm_step_planes": (C.c_int, [_P, C.c_int64, C.c_int64, C.c_int64, C.c_int, _P]),
@@ -420,6 +421,10 @@ class Lattice:
     def test_without_exchange(self):
         """Test hook: frees what the lattice's tiles exchange (see lbm_test_without_exchange)."""
         _check(lib().lbm_test_without_exchange(self._h))
+
+    def test_refuse_rounds(self, on: bool = True):
+        """Test hook: launches in rounds are refused as where their CTAs cannot all be resident (see lbm_test_refuse_rounds)."""
+        _check(lib().lbm_test_refuse_rounds(self._h, int(bool(on))))
 
     def test_last_tiles(self):
         """Test hook: (shape, rows, steps, rounds) of the last run's tiles (see lbm_test_last_tiles); shape 0: none."""

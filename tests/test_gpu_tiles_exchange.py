@@ -34,6 +34,42 @@ def test_without_memory_for_the_exchange(nx, ny, storage):
         assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
 
 
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("nx,ny,storage", [(128, 128, lb.F32), (180, 164, lb.F16S), (301, 199, lb.F64)])
+def test_where_the_ctas_cannot_all_be_resident(nx, ny, storage, captured):
+    """A refused launch in rounds is made again as one launch per few steps, in the same run and with the same results, also
+    where a captured run has fixed the parity of the buffers; rounds come back once they are launched."""
+    with lattice(nx, ny, storage) as lat, lattice(nx, ny, storage, lb.KERNEL_PLAIN) as ref:
+        lat.step(31)
+        done = 31
+        if captured:
+            torch = pytest.importorskip("torch")
+            stream = torch.cuda.Stream()
+            lat.set_stream(stream)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                lat.step(2)
+        for refused in (True, False):
+            lat.test_refuse_rounds(refused)
+            for n in (30, 31, 46):
+                at = lat.device_populations()[0]
+                lat.step(n)
+                done += n
+                shape, _, _, rounds = lat.test_last_tiles()
+                assert shape in (1, 2) and rounds == (0 if refused else 1)
+                if captured and n % 2 == 0:
+                    assert lat.device_populations()[0] == at
+                lat.sync()
+        if captured:
+            with torch.cuda.stream(stream):
+                graph.replay()
+            torch.cuda.synchronize()
+            done += 2
+            del graph
+        ref.step(done)
+        assert np.array_equal(lat.get_populations(np.float64), ref.get_populations(np.float64))
+
+
 TIMEOUT = -8
 
 
